@@ -1,17 +1,25 @@
-// Warp-level FFT of length G = 32*P (P in {4, 8, 16, 32}, or R times such a length for
-// R in {3, 5}; see FftPlan) in FP32 registers.
+// Line FFT of length G over C interleaved sequences, by the threads of one CTA in FP32.
 //
-// One warp transforms one G-point sequence held as P values per lane
-// (lane l, register j <-> element l + 32 j). Four-step decomposition G = P x 32:
-//   1. P-point DFT over j in registers (radix-2 DIT, compile-time twiddles),
-//   2. twiddle W_G^(l k),
-//   3. transpose through a padded per-warp shared buffer,
-//   4. 32-point DFTs over l, each split across T = 32/P lanes: a P-point register DFT
-//      per lane, twiddle W_32^(h m), then a T-point DFT across the T lanes by shuffles.
-// Output: lane (k = lane / T, h = lane % T) holds X[k + P q + P^2 k3] in register m, with
-// (q, k3) from the cross-lane step (warp_fft_pow2_out_index).
-// Forward = exp(-2 pi i nk/G), inverse = exp(+2 pi i nk/G), both unnormalized.
-// Twiddles are FP64-computed, FP32-stored tables (host fills them once per plan).
+// A line is [G][C] complex, coil fastest. Thread t works for coil t % C; a pass is a set of
+// independent radix-R butterflies, taken TB at a time (TB = threads / C), so neighbouring
+// threads touch neighbouring memory in global and in shared memory alike. G = R1 R2 R3:
+//   1. radix R1 over n = b + S1 j (j < R1, S1 = G / R1), straight from the caller's load(n)
+//      (global memory; zero padding costs no read), times W_G^(b k1), to shared row
+//      b + S1 k1;
+//   2. radix R2 inside each k1 block, in place, times W_S1^(b2 k2);
+//   3. radix R3, straight to the caller's store(k): X[k1 + R1 k2 + R1 R2 k3].
+// G = R1 R2 skips the middle pass. A butterfly of a pass reads and writes the same rows, so a
+// pass needs no registers beyond one butterfly and one barrier separates two passes. Each k1
+// block is followed by one pad row: the last pass reads rows S1 + 1 apart, an odd number of
+// rows, which spreads them over the banks.
+//
+// What bounds it: shared-memory bandwidth and instruction issue, beside the line's own global
+// traffic. The passes move each value through shared memory once (two radices) or twice
+// (three). It replaces a warp-per-coil FFT that staged slabs, transposes and outputs through
+// shared memory (four round trips per value, 1130 warp instructions per 512-point FFT).
+//
+// Forward = exp(-2 pi i nk/G), inverse = exp(+2 pi i nk/G), both unnormalized. tw is the
+// plan's table exp(-2 pi i e / G), FP64-computed and FP32-stored.
 // The reference's FFT endpoints are SIMT FP32 shared-memory radix-8/16/32 kernels
 // (nufft_custom_fft_forward_bench.cu:918-999, :1463-1552); this is an independent design.
 #pragma once
@@ -21,294 +29,257 @@
 namespace tsn {
 namespace dev {
 
-// exp(-2 pi i e / 1024), e in [0, 1024); defined here, filled once per process by the host.
-// (included by exactly one translation unit)
-__constant__ float2 c_w1024[1024];
-
-// exp(-2 pi i j / R) for R = 3 and 5, filled with the plan twiddle tables' FP64 expression
-// (so equal to tw[B j] of a G = R B plan): uniform across lanes, read as constant operands
-__constant__ float2 c_wr3[3];
-__constant__ float2 c_wr5[5];
-
-template <int R, bool INV>
-__device__ __forceinline__ float2 radix_twiddle(int j) {
-  const float2 w = R == 3 ? c_wr3[j] : c_wr5[j];
-  return INV ? make_float2(w.x, -w.y) : w;
+// multiply by exp(-i pi / 2) (forward) or exp(+i pi / 2) (inverse)
+template <bool INV>
+__host__ __device__ __forceinline__ float2 rot90(float2 a) {
+  return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
+// multiply by (c, -s) (forward) or (c, +s) (inverse)
+template <bool INV>
+__host__ __device__ __forceinline__ float2 rot(float2 a, float c, float s) {
+  return INV ? make_float2(a.x * c - a.y * s, a.y * c + a.x * s) : make_float2(a.x * c + a.y * s, a.y * c - a.x * s);
+}
+
+// In-register DFT of length R, natural order in and out.
+template <int R, bool INV>
+struct Dft;
 
 template <bool INV>
-__device__ __forceinline__ float2 const_twiddle(int e1024) {
-  const float2 w = c_w1024[e1024 & 1023];
-  return INV ? make_float2(w.x, -w.y) : w;
-}
+struct Dft<2, INV> {
+  static __host__ __device__ __forceinline__ void run(float2& a, float2& b) {
+    const float2 t = a;
+    a = cadd(t, b);
+    b = csub(t, b);
+  }
+};
 
-__host__ __device__ constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
-__host__ __device__ constexpr int bitrev(int x, int bits) {
-  return bits == 0 ? 0 : (((x & 1) << (bits - 1)) | bitrev(x >> 1, bits - 1));
-}
+template <bool INV>
+struct Dft<3, INV> {
+  static __host__ __device__ __forceinline__ void run(float2& a, float2& b, float2& c) {
+    const float h = 0.86602540378443864676f;  // sin(pi/3)
+    const float2 s = cadd(b, c), d = cscale(rot90<INV>(csub(b, c)), h);
+    const float2 m = make_float2(a.x - 0.5f * s.x, a.y - 0.5f * s.y);
+    a = cadd(a, s);
+    b = cadd(m, d);
+    c = csub(m, d);
+  }
+};
 
-// One radix-2 DIT stage of butterfly span LEN, then the next stage (compile-time
-// recursion keeps every register index a constant, so the array never spills to
-// local memory).
-template <int P, bool INV, int LEN>
-struct DitStage {
-  static __device__ __forceinline__ void run(float2 (&a)[P]) {
-    constexpr int HALF = LEN / 2;
+template <bool INV>
+struct Dft<4, INV> {
+  static __host__ __device__ __forceinline__ void run(float2& a, float2& b, float2& c, float2& d) {
+    const float2 s0 = cadd(a, c), d0 = csub(a, c), s1 = cadd(b, d), d1 = rot90<INV>(csub(b, d));
+    a = cadd(s0, s1);
+    b = cadd(d0, d1);
+    c = csub(s0, s1);
+    d = csub(d0, d1);
+  }
+};
+
+template <bool INV>
+struct Dft<5, INV> {
+  static __host__ __device__ __forceinline__ void run(float2& a, float2& b, float2& c, float2& d, float2& e) {
+    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;  // cos(2 pi/5), cos(4 pi/5)
+    const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;   // sin(2 pi/5), sin(4 pi/5)
+    const float2 p1 = cadd(b, e), m1 = rot90<INV>(csub(b, e)), p2 = cadd(c, d), m2 = rot90<INV>(csub(c, d));
+    const float2 u1 = make_float2(a.x + c1 * p1.x + c2 * p2.x, a.y + c1 * p1.y + c2 * p2.y);
+    const float2 u2 = make_float2(a.x + c2 * p1.x + c1 * p2.x, a.y + c2 * p1.y + c1 * p2.y);
+    const float2 v1 = make_float2(s1 * m1.x + s2 * m2.x, s1 * m1.y + s2 * m2.y);
+    const float2 v2 = make_float2(s2 * m1.x - s1 * m2.x, s2 * m1.y - s1 * m2.y);
+    a = make_float2(a.x + p1.x + p2.x, a.y + p1.y + p2.y);
+    b = cadd(u1, v1);
+    c = cadd(u2, v2);
+    d = csub(u2, v2);
+    e = csub(u1, v1);
+  }
+};
+
+// Length 6 and 10 = 2 * odd, coprime factors (no twiddles): element n = (P n1 + 2 n2) mod R,
+// output k = the index with k mod 2 = k1, k mod P = k2.
+template <bool INV>
+struct Dft<6, INV> {
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[6]) {
+    float2 a[3] = {v[0], v[2], v[4]}, b[3] = {v[3], v[5], v[1]};
+    Dft<3, INV>::run(a[0], a[1], a[2]);
+    Dft<3, INV>::run(b[0], b[1], b[2]);
 #pragma unroll
-    for (int i = 0; i < P; i += LEN) {
+    for (int k = 0; k < 3; ++k) Dft<2, INV>::run(a[k], b[k]);
+    // The length-3 output index is 2 k2 mod 3 of the decimated transform: k2 = 0, 1, 2 of a
+    // belongs to k = 0, 4, 2 (even) and b to k = 3, 1, 5 (odd)
+    v[0] = a[0]; v[4] = a[1]; v[2] = a[2];
+    v[3] = b[0]; v[1] = b[1]; v[5] = b[2];
+  }
+};
+
+template <bool INV>
+struct Dft<10, INV> {
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[10]) {
+    float2 a[5] = {v[0], v[2], v[4], v[6], v[8]}, b[5] = {v[5], v[7], v[9], v[1], v[3]};
+    Dft<5, INV>::run(a[0], a[1], a[2], a[3], a[4]);
+    Dft<5, INV>::run(b[0], b[1], b[2], b[3], b[4]);
 #pragma unroll
-      for (int j = 0; j < HALF; ++j) {
-        const float2 u = a[i + j];
-        float2 t = a[i + j + HALF];
-        if (j != 0) {
-          if (4 * j == LEN) {  // W_LEN^(LEN/4) = -i (forward) / +i (inverse)
-            t = INV ? make_float2(-t.y, t.x) : make_float2(t.y, -t.x);
-          } else {
-            t = cmul(const_twiddle<INV>(j * (1024 / LEN)), t);
-          }
+    for (int k = 0; k < 5; ++k) Dft<2, INV>::run(a[k], b[k]);
+    // even k = k2 mod 5: 0, 6, 2, 8, 4; odd k: 5, 1, 7, 3, 9
+    v[0] = a[0]; v[6] = a[1]; v[2] = a[2]; v[8] = a[3]; v[4] = a[4];
+    v[5] = b[0]; v[1] = b[1]; v[7] = b[2]; v[3] = b[3]; v[9] = b[4];
+  }
+};
+
+template <bool INV>
+struct Dft<8, INV> {
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[8]) {
+    const float h = 0.70710678118654752440f;
+    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    Dft<4, INV>::run(e[0], e[1], e[2], e[3]);
+    Dft<4, INV>::run(o[0], o[1], o[2], o[3]);
+    // o[k] *= W_8^k
+    o[1] = cscale(INV ? make_float2(o[1].x - o[1].y, o[1].y + o[1].x) : make_float2(o[1].x + o[1].y, o[1].y - o[1].x), h);
+    o[2] = rot90<INV>(o[2]);
+    o[3] = cscale(INV ? make_float2(-o[3].x - o[3].y, o[3].x - o[3].y) : make_float2(o[3].y - o[3].x, -o[3].x - o[3].y), h);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = cadd(e[k], o[k]);
+      v[k + 4] = csub(e[k], o[k]);
+    }
+  }
+};
+
+template <bool INV>
+struct Dft<16, INV> {
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[16]) {
+    const float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f;  // cos, sin of pi/8
+    const float h = 0.70710678118654752440f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) Dft<4, INV>::run(v[i], v[i + 4], v[i + 8], v[i + 12]);
+    // v[i + 4 k] *= W_16^(i k)
+    v[5] = rot<INV>(v[5], c1, s1);
+    v[6] = rot<INV>(v[6], h, h);
+    v[7] = rot<INV>(v[7], s1, c1);
+    v[9] = rot<INV>(v[9], h, h);
+    v[10] = rot90<INV>(v[10]);
+    v[11] = rot<INV>(v[11], -h, h);
+    v[13] = rot<INV>(v[13], s1, c1);
+    v[14] = rot<INV>(v[14], -h, h);
+    v[15] = rot<INV>(v[15], -c1, -s1);
+    float2 o[16];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      Dft<4, INV>::run(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[k + 4 * q] = v[4 * k + q];
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = o[k];
+  }
+};
+
+// Radices of each supported length.
+template <int G>
+struct FftRadix;
+template <> struct FftRadix<128> { static constexpr int R1 = 8, R2 = 16, R3 = 1, TB = 16; };
+template <> struct FftRadix<256> { static constexpr int R1 = 16, R2 = 16, R3 = 1, TB = 16; };
+template <> struct FftRadix<384> { static constexpr int R1 = 8, R2 = 8, R3 = 6, TB = 16; };
+template <> struct FftRadix<512> { static constexpr int R1 = 8, R2 = 8, R3 = 8, TB = 32; };
+template <> struct FftRadix<640> { static constexpr int R1 = 8, R2 = 8, R3 = 10, TB = 40; };
+template <> struct FftRadix<1024> { static constexpr int R1 = 16, R2 = 8, R3 = 8, TB = 64; };
+
+// C: interleaved sequences in shared memory (coils of this CTA)
+template <int G, int C, bool INV>
+struct LineFft {
+  using P = FftRadix<G>;
+  static constexpr int R1 = P::R1, R2 = P::R2, R3 = P::R3, TB = P::TB;
+  static constexpr int THREADS = C * TB;
+  static constexpr int S1 = G / R1, S2 = S1 / R2;
+  static constexpr int RL = R3 > 1 ? R3 : R2;     // radix of the last pass
+  static constexpr int NL = G / RL;               // butterflies of the last pass
+  static constexpr int ITL = (NL + TB - 1) / TB;  // its iterations per thread
+  static constexpr int ROWS = G + R1;             // shared rows of C complex values
+  static_assert(R1 * R2 * R3 == G, "radices");
+
+  static __host__ __device__ __forceinline__ float2 twiddle(float2 v, const float2* tw, int e) {
+    const float2 w = tw[e];
+    return INV ? cmulc(v, w) : cmul(v, w);
+  }
+
+  // load(n): element n of the line, 0 <= n < G
+  template <class Load>
+  static __host__ __device__ __forceinline__ void first(float2* s, const float2* tw, int tid, Load load) {
+    constexpr int IT = (S1 + TB - 1) / TB;
+    constexpr int GROUP = R1 >= 16 ? 1 : 2;  // butterflies whose loads are in flight together
+    const int c = tid % C, b0 = tid / C;
+#pragma unroll
+    for (int i0 = 0; i0 < IT; i0 += GROUP) {
+      float2 v[GROUP][R1];
+#pragma unroll
+      for (int g = 0; g < GROUP; ++g) {
+        const int b = b0 + (i0 + g) * TB;
+        if (i0 + g < IT && (S1 % TB == 0 || b < S1)) {
+#pragma unroll
+          for (int j = 0; j < R1; ++j) v[g][j] = load(b + S1 * j);
         }
-        a[i + j] = cadd(u, t);
-        a[i + j + HALF] = csub(u, t);
-      }
-    }
-    DitStage<P, INV, LEN * 2>::run(a);
-  }
-};
-template <int P, bool INV>
-struct DitStage<P, INV, 2 * P> {
-  static __device__ __forceinline__ void run(float2 (&)[P]) {}
-};
-
-template <int P, int I>
-struct BitReverse {
-  static __device__ __forceinline__ void run(float2 (&a)[P]) {
-    constexpr int J = bitrev(I, ilog2(P));
-    if constexpr (J > I) {
-      const float2 t = a[I];
-      a[I] = a[J];
-      a[J] = t;
-    }
-    BitReverse<P, I + 1>::run(a);
-  }
-};
-template <int P>
-struct BitReverse<P, P> {
-  static __device__ __forceinline__ void run(float2 (&)[P]) {}
-};
-
-// In-register DFT of length P (power of two), natural order in and out.
-template <int P, bool INV>
-__device__ __forceinline__ void dft_reg(float2 (&a)[P]) {
-  BitReverse<P, 0>::run(a);
-  DitStage<P, INV, 2>::run(a);
-}
-
-template <int G>
-struct WarpFftShape {
-  static constexpr int P = G / 32;
-  static constexpr int T = 32 / P;
-  static constexpr int PITCH = 32 + T;        // padded row pitch (float2) of the transpose buffer
-  static constexpr int SCRATCH = P * PITCH;   // float2 per warp
-  static_assert(P * 32 == G && (P & (P - 1)) == 0 && P >= 4 && P <= 32, "G must be 32*P, P in {4..32}");
-};
-
-// Power-of-two warp FFT. tw: shared table exp(-2 pi i e / (G * TS)), e in [0, G * TS); the
-// transform reads every TS-th entry (TS > 1 when it is the base of a mixed-radix length).
-template <int G, bool INV, int TS = 1>
-__device__ __forceinline__ void warp_fft_pow2(float2 (&v)[G / 32], float2* scratch, const float2* tw) {
-  using S = WarpFftShape<G>;
-  constexpr int P = S::P, T = S::T;
-  const int lane = threadIdx.x & 31;
-  dft_reg<P, INV>(v);
-  // twiddles W_G^(lane k): the power-of-two exponents come from the table, the others are
-  // products of at most three of them (W^k = W^(high bit of k) W^(rest)), which trades shared
-  // memory loads for FP32 multiplies at an error of a few ulp
-  {
-    float2 wk[P];
-    wk[0] = make_float2(1.f, 0.f);
-#pragma unroll
-    for (int k = 1; k < P; ++k) {
-      if ((k & (k - 1)) == 0) {
-        wk[k] = tw[TS * ((lane * k) & (G - 1))];
-        if (INV) wk[k].y = -wk[k].y;
-      } else {
-        const int hb = 1 << (31 - __clz(k));
-        wk[k] = cmul(wk[hb], wk[k - hb]);
-      }
-      v[k] = cmul(v[k], wk[k]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < P; ++k) scratch[k * S::PITCH + lane] = v[k];
-  __syncwarp();
-  const int kk = lane / T, h = lane % T;
-#pragma unroll
-  for (int i = 0; i < P; ++i) v[i] = scratch[kk * S::PITCH + T * i + h];
-  __syncwarp();
-  dft_reg<P, INV>(v);
-  if (T > 1) {
-#pragma unroll
-    for (int m = 1; m < P; ++m) {
-      float2 w = tw[TS * ((h * m * P) & (G - 1))];
-      if (INV) w.y = -w.y;
-      v[m] = cmul(v[m], w);
-    }
-    if (T == 2) {
-#pragma unroll
-      for (int m = 0; m < P; ++m) {
-        float2 o;
-        o.x = __shfl_xor_sync(0xFFFFFFFFu, v[m].x, 1);
-        o.y = __shfl_xor_sync(0xFFFFFFFFu, v[m].y, 1);
-        v[m] = h == 0 ? cadd(v[m], o) : csub(o, v[m]);
-      }
-    } else if (T == 4) {
-      // The 4-point DFTs across lanes go through the warp scratch instead of shuffles: lane
-      // (kk, h) takes the Q = P/4 columns m = h Q + i and, for each, the values of the four
-      // lanes kk*4 + h2. Rows are XOR-swizzled by the column group m / Q, which makes both the
-      // row writes and these reads conflict-free. Then a register DFT-4 per column.
-      constexpr int Q = P / 4;
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < P; ++m) scratch[m * 32 + (lane ^ (m / Q))] = v[m];
-      __syncwarp();
-      float2 u[Q][4];
-#pragma unroll
-      for (int i = 0; i < Q; ++i)
-#pragma unroll
-        for (int h2 = 0; h2 < 4; ++h2) u[i][h2] = scratch[(h * Q + i) * 32 + ((kk * 4 + h2) ^ h)];
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < Q; ++i) {
-        dft_reg<4, INV>(u[i]);
-#pragma unroll
-        for (int k3 = 0; k3 < 4; ++k3) v[i * 4 + k3] = u[i][k3];
-      }
-    } else {
-      // T == 8 (P == 4): each 8-point DFT across lanes is split over a lane pair. Lane (kk, h)
-      // takes column m = h / 2 and the four values of lanes kk*8 + 2 j + e (e = h % 2) from the
-      // scratch (XOR swizzle 2m: conflict-free), a register DFT-4 gives the even (e = 0) or odd
-      // (e = 1) half, the odd half is multiplied by W_8^k, and one shuffle exchange across the
-      // pair forms X[k] = E[k] + W_8^k O[k] (e = 0) and X[k + 4] = E[k] - W_8^k O[k] (e = 1).
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < P; ++m) scratch[m * 32 + (lane ^ (2 * m))] = v[m];
-      __syncwarp();
-      const int mm = h >> 1, e = h & 1;
-      float2 u[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) u[j] = scratch[mm * 32 + ((kk * 8 + 2 * j + e) ^ (2 * mm))];
-      __syncwarp();
-      dft_reg<4, INV>(u);
-#pragma unroll
-      for (int k = 1; k < 4; ++k)
-        if (e) u[k] = cmul(u[k], const_twiddle<INV>(k * 128));  // W_8^k = exp(-2 pi i k / 8)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        float2 o;
-        o.x = __shfl_xor_sync(0xFFFFFFFFu, u[k].x, 1);
-        o.y = __shfl_xor_sync(0xFFFFFFFFu, u[k].y, 1);
-        v[k] = e ? csub(o, u[k]) : cadd(u[k], o);
-      }
-    }
-  }
-}
-
-// Output element index held in register m after warp_fft_pow2<G>: lane (kk = lane / T,
-// h = lane % T) holds X[kk + P q + P^2 k3] with, by the cross-lane step,
-//   T <= 2: q = m, k3 = h;
-//   T == 4: q = h (P/4) + m / 4, k3 = m % 4;
-//   T == 8: q = h / 2, k3 = m + 4 (h % 2).
-template <int G>
-__device__ __forceinline__ int warp_fft_pow2_out_index(int m) {
-  using S = WarpFftShape<G>;
-  constexpr int P = S::P, T = S::T;
-  const int lane = threadIdx.x & 31;
-  const int kk = lane / T, h = lane % T;
-  if constexpr (T == 4) return kk + P * (h * (P / 4) + m / 4) + P * P * (m % 4);
-  else if constexpr (T == 8) return kk + P * (h >> 1) + P * P * (m + 4 * (h & 1));
-  else return kk + P * m + P * P * h;
-}
-
-// Lengths G = R * B with R in {1, 3, 5} and a power-of-two base B = 32 * 2^k >= 128; the
-// radix-3 and radix-5 factors give the grids 2N of image sizes N = 192 and 320.
-template <int G>
-struct FftPlan {
-  static constexpr int R = (G % 5 == 0) ? 5 : (G % 3 == 0) ? 3 : 1;
-  static constexpr int B = G / R;                           // power-of-two base length
-  static constexpr int P = G / 32;                          // registers per lane
-  static constexpr int PB = B / 32;                         // registers per lane of one base FFT
-  static constexpr int SCRATCH = WarpFftShape<B>::SCRATCH;  // float2 per warp
-};
-
-// Input element held in register j before warp_fft: lane + 32 j for power-of-two lengths;
-// for G = R B, register r * PB + j' holds x[R (lane + 32 j') + r] (decimation by R).
-template <int G>
-__device__ __forceinline__ int warp_fft_in_index(int j) {
-  using F = FftPlan<G>;
-  const int lane = threadIdx.x & 31;
-  if constexpr (F::R == 1) return lane + 32 * j;
-  else return F::R * (lane + 32 * (j % F::PB)) + j / F::PB;
-}
-
-// Output element index held in register m after warp_fft.
-template <int G>
-__device__ __forceinline__ int warp_fft_out_index(int m) {
-  using F = FftPlan<G>;
-  if constexpr (F::R == 1) return warp_fft_pow2_out_index<G>(m);
-  else return warp_fft_pow2_out_index<F::B>(m % F::PB) + F::B * (m / F::PB);
-}
-
-// Warp FFT of length G (see FftPlan). tw: shared table exp(-2 pi i e / G), e in [0, G).
-// For G = R B: R base FFTs of the decimated sequences Y_r, then for each base output k a
-// radix-R step in registers, X[k + B q] = sum_r W_G^{r k} Y_r[k] W_R^{r q}.
-template <int G, bool INV>
-__device__ __forceinline__ void warp_fft(float2 (&v)[G / 32], float2* scratch, const float2* tw) {
-  using F = FftPlan<G>;
-  if constexpr (F::R == 1) {
-    warp_fft_pow2<G, INV>(v, scratch, tw);
-  } else {
-    constexpr int R = F::R, B = F::B, PB = F::PB;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float2 sub[PB];
-#pragma unroll
-      for (int j = 0; j < PB; ++j) sub[j] = v[r * PB + j];
-      warp_fft_pow2<B, INV, R>(sub, scratch, tw);  // W_B^e = tw[R e]
-#pragma unroll
-      for (int j = 0; j < PB; ++j) v[r * PB + j] = sub[j];
-    }
-#pragma unroll
-    for (int m = 0; m < PB; ++m) {
-      const int k = warp_fft_pow2_out_index<B>(m);
-      float2 t[R];
-      t[0] = v[m];
-      // W_G^(r k), r < R: W^k and (R == 5) W^2k from the table, the rest as products
-      float2 wr[R];
-      wr[1] = tw[k];
-      if (INV) wr[1].y = -wr[1].y;
-      if constexpr (R == 3) {
-        wr[2] = cmul(wr[1], wr[1]);
-      } else {
-        wr[2] = tw[2 * k];  // 2 k < G
-        if (INV) wr[2].y = -wr[2].y;
-        wr[3] = cmul(wr[2], wr[1]);
-        wr[4] = cmul(wr[2], wr[2]);
       }
 #pragma unroll
-      for (int r = 1; r < R; ++r) t[r] = cmul(v[r * PB + m], wr[r]);
+      for (int g = 0; g < GROUP; ++g) {
+        const int b = b0 + (i0 + g) * TB;
+        if (i0 + g < IT && (S1 % TB == 0 || b < S1)) {
+          Dft<R1, INV>::run(v[g]);
+          s[b * C + c] = v[g][0];
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        float2 acc = t[0];
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          const float2 w = radix_twiddle<R, INV>((r * q) % R);  // W_R^{r q}, a constant operand
-          acc = cadd(acc, cmul(t[r], w));
+          for (int k = 1; k < R1; ++k) s[(b + (S1 + 1) * k) * C + c] = twiddle(v[g][k], tw, b * k);
         }
-        v[q * PB + m] = acc;
       }
     }
   }
-}
+
+  // middle pass of a three-radix length
+  static __host__ __device__ __forceinline__ void middle(float2* s, const float2* tw, int tid) {
+    if constexpr (R3 > 1) {
+      constexpr int NB = R1 * S2, IT = (NB + TB - 1) / TB;
+      const int c = tid % C, b0 = tid / C;
+#pragma unroll
+      for (int i = 0; i < IT; ++i) {
+        const int b = b0 + i * TB;
+        if (NB % TB == 0 || b < NB) {
+          const int b2 = b % S2, k1 = b / S2;
+          float2* q = s + (b2 + (S1 + 1) * k1) * C + c;
+          float2 v[R2];
+#pragma unroll
+          for (int j = 0; j < R2; ++j) v[j] = q[S2 * j * C];
+          Dft<R2, INV>::run(v);
+          q[0] = v[0];
+#pragma unroll
+          for (int k = 1; k < R2; ++k) q[S2 * k * C] = twiddle(v[k], tw, R1 * b2 * k);
+        }
+      }
+    }
+  }
+
+  // store(i, j, k, value): output element k; i (iteration) and j are compile-time constants
+  // after unrolling, for callers that keep the values in registers
+  template <class Store>
+  static __host__ __device__ __forceinline__ void last(const float2* s, int tid, Store store) {
+    const int c = tid % C, b0 = tid / C;
+#pragma unroll
+    for (int i = 0; i < ITL; ++i) {
+      const int b = b0 + i * TB;
+      if (NL % TB == 0 || b < NL) {
+        // b = k1 + R1 k2
+        const float2* q = s + ((R3 > 1 ? RL * (b / R1) : 0) + (S1 + 1) * (b % R1)) * C + c;
+        float2 v[RL];
+#pragma unroll
+        for (int j = 0; j < RL; ++j) v[j] = q[j * C];
+        Dft<RL, INV>::run(v);
+#pragma unroll
+        for (int j = 0; j < RL; ++j) store(i, j, b + NL * j, v[j]);
+      }
+    }
+  }
+  // last-pass butterfly of iteration i of thread tid (its outputs: b + NL j), or -1
+  static __host__ __device__ __forceinline__ int last_base(int tid, int i) {
+    const int b = tid / C + i * TB;
+    return NL % TB == 0 || b < NL ? b : -1;
+  }
+};
 
 }  // namespace dev
 }  // namespace tsn

@@ -62,29 +62,6 @@ static void launch_k(void (*kernel)(KArgs...), int grid, int block, size_t smem,
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-void set_twiddle_constants(cudaStream_t s) {
-  std::vector<float2> w(1024);
-  for (int e = 0; e < 1024; ++e) {
-    const double a = -2.0 * M_PI * e / 1024.0;
-    w[e] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
-  }
-  cudaMemcpyToSymbolAsync(dev::c_w1024, w.data(), sizeof(float2) * 1024, 0, cudaMemcpyHostToDevice, s);
-  // W_R^j with the plan tables' expression (-2 pi e) / G at e = B j, G = R B: for a power-of-two
-  // B that is exactly (-2 pi j) / R, so these equal the plans' tw[B j]
-  float2 w3[3], w5[5];
-  for (int j = 0; j < 3; ++j) {
-    const double a = -2.0 * M_PI * j / 3.0;
-    w3[j] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
-  }
-  for (int j = 0; j < 5; ++j) {
-    const double a = -2.0 * M_PI * j / 5.0;
-    w5[j] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
-  }
-  cudaMemcpyToSymbolAsync(dev::c_wr3, w3, sizeof w3, 0, cudaMemcpyHostToDevice, s);
-  cudaMemcpyToSymbolAsync(dev::c_wr5, w5, sizeof w5, 0, cudaMemcpyHostToDevice, s);
-  cudaStreamSynchronize(s);
-}
-
 // ------------------------------------------------------------------------------------------
 // Sparse interpolation: one warp per 16-row group, 2:4 tiles through mma.sp m16n8k32.
 // Per tile the 32 gathered panel rows (hi and res together) are brought to shared memory
@@ -493,13 +470,8 @@ __device__ __forceinline__ double4 sum_partials4(const double* part, int nparts,
 }
 
 // ------------------------------------------------------------------------------------------
-// FFT endpoints. One warp per coil (blockDim = 32*C), one CTA per image row / grid column.
+// FFT endpoints: one CTA per line (image row, grid column) and coil group, see fft.cuh.
 // ------------------------------------------------------------------------------------------
-template <int G>
-struct FftSmem {
-  static constexpr int SCR = FftPlan<G>::SCRATCH;
-};
-
 // Copy `bytes` (multiple of 16) from global to shared with 16-byte cp.async, all threads.
 __device__ __forceinline__ void cp_async_bytes(void* dst, const void* src, int bytes) {
   uint8_t* d = static_cast<uint8_t*>(dst);
@@ -507,40 +479,26 @@ __device__ __forceinline__ void cp_async_bytes(void* dst, const void* src, int b
   for (int i = threadIdx.x * 16; i < bytes; i += blockDim.x * 16) cp_async16(d + i, q + i);
 }
 
-// [rows][C] complex slabs in shared memory hold each row's C/2 16-byte chunks XOR-swizzled
-// by the row index, so a warp reading one coil down 32 consecutive rows touches distinct
-// banks (unswizzled, 64-byte rows make that a 16-way conflict).
-__device__ __forceinline__ int slab_swz(int n, int chn) {
-  return chn == 2 ? (n >> 2) & 1 : chn == 4 ? (n >> 1) & 3 : chn == 8 ? (n & 7) : 0;
-}
-__device__ __forceinline__ int slab_idx(int n, int c, int C) {
-  return n * C + 2 * ((c >> 1) ^ slab_swz(n, C >> 1)) + (c & 1);
-}
-// copy `rows` contiguous rows of C complex values into a swizzled slab (all threads; the
-// block has 32*C threads, so every thread keeps one 16-byte chunk column, 64 rows apart)
-__device__ __forceinline__ void cp_async_slab(float2* dst, const float2* src, int rows, int C) {
-  const int chn = C >> 1;
-  const int k = threadIdx.x % chn;
-  for (int n = threadIdx.x / chn; n < rows; n += 64) cp_async16(dst + n * C + 2 * (k ^ slab_swz(n, chn)), src + n * C + 2 * k);
-}
+// CTAs per SM that the register cap leaves room for: 1024 threads at 64 registers, and for the
+// row stages, which hold a line's last butterflies and its epilogue, 768 at 80.
+#define TSN_FFT_BOUNDS(T) __launch_bounds__((T), (1024 / (T)) > 0 ? 1024 / (T) : 1)
+#define TSN_ROW_BOUNDS(T) __launch_bounds__((T), (768 / (T)) > 0 ? 768 / (T) : 1)
 
-// The four FFT stages run one warp per coil in CTAs of 32*C threads (instantiated per coil
-// count). With C <= 8 and G <= 512 the 80-register cap keeps three CTAs resident per SM (two
-// at 128 registers for larger grids). The per-warp FFT scratch and the output staging reuse
-// the input slab's shared memory once it is consumed, which keeps a CTA near 72 KB. The
-// column stages double-buffer the slab when two regions fit, so the next item streams in
-// while the current one is transformed.
-#define TSN_FFT_BOUNDS(G, MAXW) __launch_bounds__((MAXW) * 32, (MAXW) > 8 ? 1 : ((G) <= 512 ? 3 : 2))
+// Coils per CTA of the column and middle stages. 16 coils go in two CTAs of 8: a 64-byte run
+// per row is still whole sectors, and the smaller CTA halves shared memory, so that several
+// lines stay resident per SM at the largest grids. The row stages keep all coils of a line
+// together (one image update, one coil combine).
+__host__ __device__ constexpr int cols_coils(int C) { return C == 16 ? 8 : C; }
+
+// Row pitch (float2) of coil-map rows staged in shared memory for a coil-fastest reader:
+// 16 bytes off a multiple of 128, so that 8 coils of two neighbouring pixels share no bank.
+__host__ __device__ __forceinline__ int map_pitch(int N) { return (N + 15) / 16 * 16 + 2; }
 
 // Forward rows (x-stage). Image row i0 -> z1[q1][i0][c] for all q1. Fuses the SENSE
 // multiply, deapodization, power-of-two panel scaling, zero-padding and (CG) p = r + beta p.
-// Shared memory: twiddles [G] | one region that holds, in turn,
-//   the input slab  [row0 N][row1 N][maps C*N] float2 + [scaling N] float
-//     mode 0 with smaps:  row0 = x row, maps = S_c rows      (row1 unused)
-//     mode 0 without:     maps = coil-image rows
-//     mode 1 (CG):        row0 = r row, row1 = p row, maps = S_c rows
-//     mode 4 (CG, fused update): row0 = r, row1 = p, row2 = A p, row3 = x rows, maps = S_c rows
-//   the per-warp FFT scratch [C][SCR], and the output rows [G][C+1] float2.
+//   mode 0 with smaps: the row of x; without: coil-image rows
+//   mode 1 (CG): p = r + beta p, mode 2: p = r
+//   mode 4 (CG, fused update): x += alpha p, r -= alpha A p, then p = r + beta p
 // Mode 4 also finishes CG iteration iter-1, which then needs no cg_update launch: parts holds
 // four sections [lines] of <p, Ap>, Re <r, Ap>, <Ap, Ap> and <r, r> from the inverse rows, so
 // rho = <r, r> (a direct sum over the stored r, as the reference's rs_old), alpha = rho / pAp,
@@ -548,59 +506,53 @@ __device__ __forceinline__ void cp_async_slab(float2* dst, const float2* src, in
 // rounding residue clamped to 0).  The expansion restarts from the direct sum every
 // iteration, so its rounding does not accumulate while rho falls.  Each row updates
 // x += alpha p and r -= alpha Ap before p = r + beta p.
+// Shared memory: FFT rows [G + R1][C] | the line's vectors [N]: row0 = x, r or (coil images)
+// unused, later p times deapodization and panel scale; row1 = p; mode 4: row2 = A p, row3 = x |
+// deapodization [N] float | (stage_maps) coil-map rows [C][pitch]. All are copied while the
+// partial sums are reduced.
 // Reference: fft512_rows4_shared16_pad_scale<true> (nufft_custom_fft_forward_bench.cu:1600-1844);
 // the CG update of reference_sparse_solver.py:297-323.
-template <int G, int CC>
-__global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1,
-                                                     int mode, float2* __restrict__ p, float2* __restrict__ r,
-                                                     const double* __restrict__ parts, int nparts,
-                                                     CgState* __restrict__ st, int iter, float2* __restrict__ xs,
-                                                     const float2* __restrict__ ap) {
-  constexpr int P = G / 32;
+template <int G, int C>
+__global__ void TSN_ROW_BOUNDS((LineFft<G, C, false>::THREADS))
+fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1, int mode, float2* __restrict__ p,
+                float2* __restrict__ r, const double* __restrict__ parts, int nparts, CgState* __restrict__ st,
+                int iter, float2* __restrict__ xs, const float2* __restrict__ ap, int stage_maps) {
+  using F = LineFft<G, C, false>;
   extern __shared__ __align__(16) uint8_t sm[];
   const int N = f.N;
   const int lines = f.lines();
   const int64_t pix = f.pix();
-  constexpr int C = CC;  // coils (one warp each), a compile-time stride
-  const int nrow = mode == 4 ? 4 : 2;
-  const int in_f2 = (nrow + C) * N;  // float2 of the slab before the scaling row
-  float2* tw_s = reinterpret_cast<float2*>(sm);
-  uint8_t* reg = reinterpret_cast<uint8_t*>(tw_s + G);
-  float2* row0 = reinterpret_cast<float2*>(reg);
+  const bool has_beta = (mode == 1 && iter > 0) || mode == 4;
+  float2* buf = reinterpret_cast<float2*>(sm);
+  float2* row0 = buf + F::ROWS * C;
   float2* row1 = row0 + N;
-  float2* row2 = row1 + N;
-  float2* row3 = row2 + N;
-  float2* maps = row0 + nrow * N;
-  const float* srow = reinterpret_cast<const float*>(reg + in_f2 * 8);
-  float2* scr = reinterpret_cast<float2*>(reg);
-  float2* out_s = reinterpret_cast<float2*>(reg);  // [G][C+1]
+  float2* row2 = row1 + (mode >= 1 ? N : 0);
+  float2* row3 = row2 + (mode == 4 ? N : 0);
+  float* srow = reinterpret_cast<float*>(row3 + (mode == 4 ? N : 0));
+  float2* maps_s = reinterpret_cast<float2*>(srow + N);
+  const int pitch = map_pitch(N);
   __shared__ double red[132];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, c = tid % C;
   // part 1: rows no kernel of a solve writes (coil maps, deapodization); part 2: the rest
   auto issue = [&](int i0, int part) {
     const size_t off = static_cast<size_t>(i0) * N;
+    if (part & 1) {
+      cp_async_bytes(srow, f.scaling + off, N * 4);
+      if (stage_maps)
+        for (int cc = 0; cc < C; ++cc)
+          cp_async_bytes(maps_s + cc * pitch, f.smaps + static_cast<size_t>(cc) * pix + off, N * 8);
+    }
     if (part & 2) {
-      if (mode >= 1) {
-        cp_async_bytes(row0, r + off, N * 8);
-        if ((mode == 1 && iter > 0) || mode == 4) cp_async_bytes(row1, p + off, N * 8);
-        if (mode == 4) {
-          cp_async_bytes(row2, ap + off, N * 8);
-          cp_async_bytes(row3, xs + off, N * 8);
-        }
-      } else if (f.smaps) {
-        cp_async_bytes(row0, x + off, N * 8);
+      if (mode >= 1) cp_async_bytes(row0, r + off, N * 8);
+      else if (f.smaps) cp_async_bytes(row0, x + off, N * 8);
+      if (has_beta) cp_async_bytes(row1, p + off, N * 8);
+      if (mode == 4) {
+        cp_async_bytes(row2, ap + off, N * 8);
+        cp_async_bytes(row3, xs + off, N * 8);
       }
     }
-    if (part & (f.smaps ? 1 : 2)) {
-      const float2* msrc = f.smaps ? f.smaps : x;
-      for (int c = 0; c < C; ++c) cp_async_bytes(maps + c * N, msrc + static_cast<size_t>(c) * pix + off, N * 8);
-    }
-    if (part & 1) cp_async_bytes(reg + in_f2 * 8, f.scaling + off, N * 4);
     cp_async_commit();
   };
-  // the twiddles and the first item's map rows stream in while the preceding kernel drains,
-  // its other rows while the panel scale is reduced
-  cp_async_bytes(tw_s, f.tw, G * 8);
   if (blockIdx.x < lines) issue(blockIdx.x, 1);
   pdl_wait();
   pdl_trigger();
@@ -648,198 +600,123 @@ __global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) fwd_rows_kernel(FftArgs f,
   }
   const float bf = static_cast<float>(beta);
   const float scl = sigma / f.gs();
-  // output copy: C/2 16-byte chunks per grid row, 64 rows per pass of the 32*C threads
-  const int ch2 = C >> 1;
-  const int ck = threadIdx.x % ch2, crow = threadIdx.x / ch2;
+  const bool sense = f.smaps || mode >= 1;
   for (int i0 = blockIdx.x; i0 < lines; i0 += gridDim.x) {
     if (i0 != blockIdx.x) {
-      __syncthreads();  // the previous item's output rows are copied out
+      __syncthreads();  // the previous line's shared rows are read
       issue(i0, 3);
     }
+    const size_t off = static_cast<size_t>(i0) * N;
     cp_async_wait<0>();
     __syncthreads();
-    if (mode >= 1) {  // p = r + beta p (p = r at iteration 0 and after a restart); row0 becomes p
-      for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const size_t px = static_cast<size_t>(i0) * N + i;
-        float2 pv = row0[i];
-        if (mode == 4) {  // x += alpha p, r -= alpha Ap (the previous iteration's update)
-          const float2 po = row1[i], av = row2[i], xv = row3[i];
-          pv.x -= af * av.x;
-          pv.y -= af * av.y;
-          r[px] = pv;
-          xs[px] = make_float2(xv.x + af * po.x, xv.y + af * po.y);
-        }
-        if ((mode == 1 && iter > 0) || mode == 4) {
-          const float2 po = row1[i];
-          pv = make_float2(pv.x + bf * po.x, pv.y + bf * po.y);
-        }
-        row0[i] = pv;
-        p[px] = pv;
+    for (int i = tid; i < N; i += F::THREADS) {
+      const float d = srow[i] * scl;
+      if (!sense) {
+        row0[i].x = d;
+        continue;
       }
-      __syncthreads();
+      float2 v = row0[i];
+      if (has_beta) {
+        const float2 pv = row1[i];
+        if (mode == 4) {  // x += alpha p, r -= alpha Ap (the previous iteration's update)
+          const float2 av = row2[i], xv = row3[i];
+          v.x -= af * av.x;
+          v.y -= af * av.y;
+          r[off + i] = v;
+          xs[off + i] = make_float2(xv.x + af * pv.x, xv.y + af * pv.y);
+        }
+        v = make_float2(v.x + bf * pv.x, v.y + bf * pv.y);
+      }
+      if (mode >= 1) p[off + i] = v;
+      row0[i] = cscale(v, d);
     }
-    float2 v[P];
-    const int c = warp;
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int n = warp_fft_in_index<G>(j);
+    __syncthreads();
+    const float2* msrc = stage_maps ? maps_s + c * pitch : (f.smaps ? f.smaps : x) + static_cast<size_t>(c) * pix + off;
+    F::first(buf, f.tw, tid, [&](int n) {
       int i1 = n + f.shift;
       if (i1 >= G) i1 -= G;
-      float2 val = make_float2(0.f, 0.f);
-      if (i1 < N) {
-        const float d = srow[i1] * scl;
-        val = (f.smaps || mode >= 1) ? cscale(cmul(row0[i1], maps[c * N + i1]), d) : cscale(maps[c * N + i1], d);
-      }
-      v[j] = val;
-    }
-    __syncthreads();  // slab consumed: the region becomes FFT scratch
-    warp_fft<G, false>(v, scr + c * FftSmem<G>::SCR, tw_s);
-    __syncthreads();  // scratch free: the region becomes the output rows
-#pragma unroll
-    for (int m = 0; m < P; ++m) out_s[warp_fft_out_index<G>(m) * (C + 1) + c] = v[m];
+      if (i1 >= N) return make_float2(0.f, 0.f);
+      const float2 w = row0[i1];
+      return sense ? cmul(w, msrc[i1]) : cscale(msrc[i1], w.x);
+    });
     __syncthreads();
-    // line i0 = (slab, row): z1 [slab][q][row][c] (one slab for images)
-    const size_t obase = static_cast<size_t>(i0 / N) * G * N + i0 % N;
-    for (int q1 = crow; q1 < G; q1 += 64) {
-      const float2 a = out_s[q1 * (C + 1) + 2 * ck], b = out_s[q1 * (C + 1) + 2 * ck + 1];
-      *reinterpret_cast<float4*>(z1 + (obase + static_cast<size_t>(q1) * N) * C + 2 * ck) = make_float4(a.x, a.y, b.x, b.y);
+    if constexpr (F::R3 > 1) {
+      F::middle(buf, f.tw, tid);
+      __syncthreads();
     }
+    // line i0 = (slab, row): z1 [slab][q][row][c] (one slab for images)
+    float2* dst = z1 + (static_cast<size_t>(i0 / N) * G * N + i0 % N) * C + c;
+    F::last(buf, tid, [&](int, int, int k, float2 v) { dst[static_cast<size_t>(k) * N * C] = v; });
   }
 }
 
 // Forward columns (y-stage): z1[q1][*][c] -> panel rows q1*G + q0, FP16 hi | res.
-// Shared memory: twiddles [G] | nbuf regions of `region` bytes, each holding in turn the
-// swizzled input slab [N][C], the per-warp FFT scratch and the output rows [G][2C+1] words.
+// Shared memory: FFT rows [G + R1][coils of the CTA].
 // Reference: fft512_allcoils1_shared16_to_n16 (nufft_custom_fft_forward_bench.cu:538-747).
-template <int G, int CC>
-__global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) fwd_cols_kernel(FftArgs f, const float2* __restrict__ z1,
-                                                     __half* __restrict__ panel, int region, int nbuf) {
-  constexpr int P = G / 32;
+template <int G, int C>
+__global__ void TSN_FFT_BOUNDS((LineFft<G, cols_coils(C), false>::THREADS))
+fwd_cols_kernel(FftArgs f, const float2* __restrict__ z1, __half* __restrict__ panel) {
+  constexpr int CC = cols_coils(C), GROUPS = C / CC;
+  using F = LineFft<G, CC, false>;
   extern __shared__ __align__(16) uint8_t sm[];
-  const int N = f.N;
-  constexpr int C = CC;  // coils (one warp each), a compile-time stride
-  float2* tw_s = reinterpret_cast<float2*>(sm);
-  uint8_t* regs = reinterpret_cast<uint8_t*>(tw_s + G);
-  const int OP = 2 * C + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto issue = [&](int q1, int b) {
-    cp_async_slab(reinterpret_cast<float2*>(regs + b * region), z1 + static_cast<size_t>(q1) * N * C, N, C);
-    cp_async_commit();
-  };
-  const int items = f.gcols();
-  cp_async_bytes(tw_s, f.tw, G * 8);
+  float2* buf = reinterpret_cast<float2*>(sm);
+  const int N = f.N, items = f.gcols() * GROUPS;
   pdl_wait();
   pdl_trigger();
-  if (blockIdx.x < items) issue(blockIdx.x, 0);
-  const int ch2 = C >> 1;  // 16-byte chunks per panel row
-  const int ck = threadIdx.x % ch2, crow = threadIdx.x / ch2;
-  const int c = warp;
-  const int lane_off = 2 * ((c >> 1) ^ slab_swz(lane + f.shift, C >> 1)) + (c & 1);
-  int it = 0;
-  for (int q1 = blockIdx.x; q1 < items; q1 += gridDim.x, ++it) {
-    const int b = nbuf == 2 ? (it & 1) : 0;
-    if (nbuf == 1 && it > 0) {
-      __syncthreads();  // the previous item's output rows are copied out
-      issue(q1, 0);
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    if (nbuf == 2 && q1 + gridDim.x < items) issue(q1 + gridDim.x, b ^ 1);
-    uint8_t* reg = regs + b * region;
-    const float2* in_s = reinterpret_cast<const float2*>(reg);
-    float2 v[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int n = warp_fft_in_index<G>(j);
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+    if (it != blockIdx.x) __syncthreads();
+    const float2* src = z1 + static_cast<size_t>(q1) * N * C + c;
+    F::first(buf, f.tw, threadIdx.x, [&](int n) {
       int i0 = n + f.shift;
       if (i0 >= G) i0 -= G;
-      // power-of-two grids: the lane's low five index bits (and so its swizzle) are fixed
-      const int idx = FftPlan<G>::R == 1 ? i0 * C + lane_off : slab_idx(i0, c, C);
-      v[j] = i0 < N ? in_s[idx] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();  // slab consumed
-    warp_fft<G, false>(v, reinterpret_cast<float2*>(reg) + c * FftSmem<G>::SCR, tw_s);
-    __syncthreads();  // scratch free
-    uint32_t* out_s = reinterpret_cast<uint32_t*>(reg);
-#pragma unroll
-    for (int m = 0; m < P; ++m) {
-      const int q0 = warp_fft_out_index<G>(m);
-      uint32_t hw, rw;
-      split_hi_res2(v[m].x, v[m].y, hw, rw);
-      out_s[q0 * OP + c] = hw;
-      out_s[q0 * OP + C + c] = rw;
-    }
+      return i0 < N ? src[i0 * C] : make_float2(0.f, 0.f);
+    });
     __syncthreads();
-    uint32_t* dst = reinterpret_cast<uint32_t*>(panel + static_cast<size_t>(q1) * G * 4 * C);
-    for (int q0 = crow; q0 < G; q0 += 64) {
-      const uint32_t* s = out_s + q0 * OP + 4 * ck;
-      *reinterpret_cast<uint4*>(dst + q0 * 2 * C + 4 * ck) = make_uint4(s[0], s[1], s[2], s[3]);
+    if constexpr (F::R3 > 1) {
+      F::middle(buf, f.tw, threadIdx.x);
+      __syncthreads();
     }
+    uint32_t* dst = reinterpret_cast<uint32_t*>(panel + static_cast<size_t>(q1) * G * 4 * C) + c;
+    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+      uint32_t hw, rw;
+      split_hi_res2(v.x, v.y, hw, rw);
+      dst[k * 2 * C] = hw;
+      dst[k * 2 * C + C] = rw;
+    });
   }
 }
 
-// Forward middle axis of a volume: z1[i0][q2][i1][c] -> z2[q2][q1][i0][c]. One item per
-// (i0, q2) line: its [N][C] run of z1 is contiguous; FFT over i1 with the zero padding and
-// centring shift of the other axes; each q1 writes one 8C-byte run of z2.
-// Shared memory: twiddles [G] | nbuf regions, each holding in turn the swizzled slab [N][C],
-// the per-warp FFT scratch and the output rows [G][C+1] float2.
-template <int G, int CC>
-__global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1,
-                                                    float2* __restrict__ z2, int region, int nbuf) {
-  constexpr int P = G / 32;
+// Forward middle axis of a volume: z1[i0][q2][i1][c] -> z2[q2][q1][i0][c]. One item per line
+// (q2, i0) with i0 fastest: neighbouring CTAs write neighbouring 8C-byte runs of z2.
+// Shared memory: FFT rows [G + R1][coils of the CTA].
+template <int G, int C>
+__global__ void TSN_FFT_BOUNDS((LineFft<G, cols_coils(C), false>::THREADS))
+fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1, float2* __restrict__ z2) {
+  constexpr int CC = cols_coils(C), GROUPS = C / CC;
+  using F = LineFft<G, CC, false>;
   extern __shared__ __align__(16) uint8_t sm[];
-  const int N = f.N;
-  constexpr int C = CC;
-  const int items = N * G;
-  float2* tw_s = reinterpret_cast<float2*>(sm);
-  uint8_t* regs = reinterpret_cast<uint8_t*>(tw_s + G);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto issue = [&](int t, int b) {
-    cp_async_slab(reinterpret_cast<float2*>(regs + b * region), z1 + static_cast<size_t>(t) * N * C, N, C);
-    cp_async_commit();
-  };
-  cp_async_bytes(tw_s, f.tw, G * 8);
+  float2* buf = reinterpret_cast<float2*>(sm);
+  const int N = f.N, items = N * G * GROUPS;
   pdl_wait();
   pdl_trigger();
-  if (blockIdx.x < items) issue(blockIdx.x, 0);
-  const int ch2 = C >> 1;
-  const int ck = threadIdx.x % ch2, crow = threadIdx.x / ch2;
-  const int c = warp;
-  const int lane_off = 2 * ((c >> 1) ^ slab_swz(lane + f.shift, C >> 1)) + (c & 1);
-  int it = 0;
-  for (int t = blockIdx.x; t < items; t += gridDim.x, ++it) {
-    const int b = nbuf == 2 ? (it & 1) : 0;
-    if (nbuf == 1 && it > 0) {
-      __syncthreads();  // the previous item's output rows are copied out
-      issue(t, 0);
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    if (nbuf == 2 && t + gridDim.x < items) issue(t + gridDim.x, b ^ 1);
-    uint8_t* reg = regs + b * region;
-    const float2* in_s = reinterpret_cast<const float2*>(reg);
-    float2 v[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int n = warp_fft_in_index<G>(j);
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+    const int q2 = t / N, i0 = t - q2 * N;
+    if (it != blockIdx.x) __syncthreads();
+    const float2* src = z1 + (static_cast<size_t>(i0) * G + q2) * N * C + c;
+    F::first(buf, f.tw, threadIdx.x, [&](int n) {
       int i1 = n + f.shift;
       if (i1 >= G) i1 -= G;
-      const int idx = FftPlan<G>::R == 1 ? i1 * C + lane_off : slab_idx(i1, c, C);
-      v[j] = i1 < N ? in_s[idx] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();  // slab consumed
-    warp_fft<G, false>(v, reinterpret_cast<float2*>(reg) + c * FftSmem<G>::SCR, tw_s);
-    __syncthreads();  // scratch free
-    float2* out_s = reinterpret_cast<float2*>(reg);  // [G][C+1]
-#pragma unroll
-    for (int m = 0; m < P; ++m) out_s[warp_fft_out_index<G>(m) * (C + 1) + c] = v[m];
+      return i1 < N ? src[i1 * C] : make_float2(0.f, 0.f);
+    });
     __syncthreads();
-    const int i0 = t / G, q2 = t - (t / G) * G;
-    float2* dst = z2 + (static_cast<size_t>(q2) * G * N + i0) * C;
-    for (int q1 = crow; q1 < G; q1 += 64) {
-      const float2 a = out_s[q1 * (C + 1) + 2 * ck], bb = out_s[q1 * (C + 1) + 2 * ck + 1];
-      *reinterpret_cast<float4*>(dst + static_cast<size_t>(q1) * N * C + 2 * ck) = make_float4(a.x, a.y, bb.x, bb.y);
+    if constexpr (F::R3 > 1) {
+      F::middle(buf, f.tw, threadIdx.x);
+      __syncthreads();
     }
+    float2* dst = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
+    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) { dst[static_cast<size_t>(k) * N * C] = v; });
   }
 }
 
@@ -876,189 +753,113 @@ __global__ void split_samples_kernel(const float2* __restrict__ y, const float* 
 }
 
 // Inverse columns: grid rows q1*G + [0,G) (all coils) -> w1[q1][i0][c], i0 < N (crop).
-// Shared memory: twiddles [G] | nbuf regions, each holding in turn the swizzled slab [G][C],
-// the per-warp FFT scratch and the cropped output rows [N][C+1] float2.
+// Shared memory: FFT rows [G + R1][coils of the CTA].
 // Reference: ifft512_rows8_regular_transposed (nufft_custom_fft_forward_bench.cu:1463-1515).
-template <int G, int CC>
-__global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_cols_kernel(FftArgs f, const float2* __restrict__ grid,
-                                                     float2* __restrict__ w1, int region, int nbuf) {
-  constexpr int P = G / 32;
+template <int G, int C>
+__global__ void TSN_FFT_BOUNDS((LineFft<G, cols_coils(C), true>::THREADS))
+inv_cols_kernel(FftArgs f, const float2* __restrict__ grid, float2* __restrict__ w1) {
+  constexpr int CC = cols_coils(C), GROUPS = C / CC;
+  using F = LineFft<G, CC, true>;
   extern __shared__ __align__(16) uint8_t sm[];
-  const int N = f.N;
-  constexpr int C = CC;  // coils (one warp each), a compile-time stride
-  float2* tw_s = reinterpret_cast<float2*>(sm);
-  uint8_t* regs = reinterpret_cast<uint8_t*>(tw_s + G);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto issue = [&](int q1, int b) {
-    cp_async_slab(reinterpret_cast<float2*>(regs + b * region), grid + static_cast<size_t>(q1) * G * C, G, C);
-    cp_async_commit();
-  };
-  const int items = f.gcols();
-  cp_async_bytes(tw_s, f.tw, G * 8);
+  float2* buf = reinterpret_cast<float2*>(sm);
+  const int N = f.N, items = f.gcols() * GROUPS;
   pdl_wait();
   pdl_trigger();
-  if (blockIdx.x < items) issue(blockIdx.x, 0);
-  const int ch2 = C >> 1;  // 16-byte chunks per output row
-  const int ck = threadIdx.x % ch2, crow = threadIdx.x / ch2;
-  const int c = warp;
-  const int lane_off = 2 * ((c >> 1) ^ slab_swz(lane, C >> 1)) + (c & 1);
-  int it = 0;
-  for (int q1 = blockIdx.x; q1 < items; q1 += gridDim.x, ++it) {
-    const int b = nbuf == 2 ? (it & 1) : 0;
-    if (nbuf == 1 && it > 0) {
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+    if (it != blockIdx.x) __syncthreads();
+    const float2* src = grid + static_cast<size_t>(q1) * G * C + c;
+    F::first(buf, f.tw, threadIdx.x, [&](int n) { return src[n * C]; });
+    __syncthreads();
+    if constexpr (F::R3 > 1) {
+      F::middle(buf, f.tw, threadIdx.x);
       __syncthreads();
-      issue(q1, 0);
     }
-    cp_async_wait<0>();
-    __syncthreads();
-    if (nbuf == 2 && q1 + gridDim.x < items) issue(q1 + gridDim.x, b ^ 1);
-    uint8_t* reg = regs + b * region;
-    const float2* in_s = reinterpret_cast<const float2*>(reg);
-    float2 v[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int n = warp_fft_in_index<G>(j);
-      v[j] = in_s[FftPlan<G>::R == 1 ? n * C + lane_off : slab_idx(n, c, C)];
-    }
-    __syncthreads();
-    warp_fft<G, true>(v, reinterpret_cast<float2*>(reg) + c * FftSmem<G>::SCR, tw_s);
-    __syncthreads();
-    float2* out_s = reinterpret_cast<float2*>(reg);  // [N][C+1]
-#pragma unroll
-    for (int m = 0; m < P; ++m) {
-      int i0 = warp_fft_out_index<G>(m) + f.shift;
+    float2* dst = w1 + static_cast<size_t>(q1) * N * C + c;
+    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+      int i0 = k + f.shift;
       if (i0 >= G) i0 -= G;
-      if (i0 < N) out_s[i0 * (C + 1) + c] = v[m];
-    }
-    __syncthreads();
-    float2* dst = w1 + static_cast<size_t>(q1) * N * C;
-    for (int i0 = crow; i0 < N; i0 += 64) {
-      const float2 a = out_s[i0 * (C + 1) + 2 * ck], bb = out_s[i0 * (C + 1) + 2 * ck + 1];
-      *reinterpret_cast<float4*>(dst + i0 * C + 2 * ck) = make_float4(a.x, a.y, bb.x, bb.y);
-    }
+      if (i0 < N) dst[i0 * C] = v;
+    });
   }
 }
 
 // Inverse middle axis of a volume: z2[q2][q1][i0][c] -> z1[q2][i0][i1][c], i1 < N (crop).
-// One item per (q2, i0): G runs of C values, N*C apart, gathered into a swizzled slab; the
-// cropped output of the item is one contiguous [N][C] run.
-// Shared memory: twiddles [G] | nbuf regions, each holding in turn the slab [G][C], the
-// per-warp FFT scratch and the output rows [N][C+1] float2.
-template <int G, int CC>
-__global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_mid_kernel(FftArgs f, const float2* __restrict__ z2,
-                                                    float2* __restrict__ z1, int region, int nbuf) {
-  constexpr int P = G / 32;
+// One item per line (q2, i0), i0 fastest: neighbouring CTAs read neighbouring 8C-byte runs.
+// Shared memory: FFT rows [G + R1][coils of the CTA].
+template <int G, int C>
+__global__ void TSN_FFT_BOUNDS((LineFft<G, cols_coils(C), true>::THREADS))
+inv_mid_kernel(FftArgs f, const float2* __restrict__ z2, float2* __restrict__ z1) {
+  constexpr int CC = cols_coils(C), GROUPS = C / CC;
+  using F = LineFft<G, CC, true>;
   extern __shared__ __align__(16) uint8_t sm[];
-  const int N = f.N;
-  constexpr int C = CC;
-  const int items = G * N;
-  float2* tw_s = reinterpret_cast<float2*>(sm);
-  uint8_t* regs = reinterpret_cast<uint8_t*>(tw_s + G);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto issue = [&](int t, int b) {
-    float2* dst = reinterpret_cast<float2*>(regs + b * region);
-    const int q2 = t / N, i0 = t - (t / N) * N;
-    const float2* src = z2 + (static_cast<size_t>(q2) * G * N + i0) * C;
-    const int chn = C / 2;
-    const int k = threadIdx.x % chn;  // 32*C threads: 64 rows per pass
-    for (int q1 = threadIdx.x / chn; q1 < G; q1 += 64)
-      cp_async16(dst + q1 * C + 2 * (k ^ slab_swz(q1, chn)), src + static_cast<size_t>(q1) * N * C + 2 * k);
-    cp_async_commit();
-  };
-  cp_async_bytes(tw_s, f.tw, G * 8);
+  float2* buf = reinterpret_cast<float2*>(sm);
+  const int N = f.N, items = G * N * GROUPS;
   pdl_wait();
   pdl_trigger();
-  if (blockIdx.x < items) issue(blockIdx.x, 0);
-  const int ch2 = C >> 1;
-  const int ck = threadIdx.x % ch2, crow = threadIdx.x / ch2;
-  const int c = warp;
-  const int lane_off = 2 * ((c >> 1) ^ slab_swz(lane, C >> 1)) + (c & 1);
-  int it = 0;
-  for (int t = blockIdx.x; t < items; t += gridDim.x, ++it) {
-    const int b = nbuf == 2 ? (it & 1) : 0;
-    if (nbuf == 1 && it > 0) {
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+    const int q2 = t / N, i0 = t - q2 * N;
+    if (it != blockIdx.x) __syncthreads();
+    const float2* src = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
+    F::first(buf, f.tw, threadIdx.x, [&](int n) { return src[static_cast<size_t>(n) * N * C]; });
+    __syncthreads();
+    if constexpr (F::R3 > 1) {
+      F::middle(buf, f.tw, threadIdx.x);
       __syncthreads();
-      issue(t, 0);
     }
-    cp_async_wait<0>();
-    __syncthreads();
-    if (nbuf == 2 && t + gridDim.x < items) issue(t + gridDim.x, b ^ 1);
-    uint8_t* reg = regs + b * region;
-    const float2* in_s = reinterpret_cast<const float2*>(reg);
-    float2 v[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int n = warp_fft_in_index<G>(j);
-      v[j] = in_s[FftPlan<G>::R == 1 ? n * C + lane_off : slab_idx(n, c, C)];
-    }
-    __syncthreads();
-    warp_fft<G, true>(v, reinterpret_cast<float2*>(reg) + c * FftSmem<G>::SCR, tw_s);
-    __syncthreads();
-    float2* out_s = reinterpret_cast<float2*>(reg);  // [N][C+1]
-#pragma unroll
-    for (int m = 0; m < P; ++m) {
-      int i1 = warp_fft_out_index<G>(m) + f.shift;
+    float2* dst = z1 + static_cast<size_t>(t) * N * C + c;
+    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+      int i1 = k + f.shift;
       if (i1 >= G) i1 -= G;
-      if (i1 < N) out_s[i1 * (C + 1) + c] = v[m];
-    }
-    __syncthreads();
-    float2* dst = z1 + static_cast<size_t>(t) * N * C;
-    for (int i1 = crow; i1 < N; i1 += 64) {
-      const float2 a = out_s[i1 * (C + 1) + 2 * ck], bb = out_s[i1 * (C + 1) + 2 * ck + 1];
-      *reinterpret_cast<float4*>(dst + i1 * C + 2 * ck) = make_float4(a.x, a.y, bb.x, bb.y);
-    }
+      if (i1 < N) dst[i1 * C] = v;
+    });
   }
 }
 
 // Inverse rows + crop + deapodization + SENSE coil combine (+ CG epilogues).
-// Shared memory: twiddles [G] | a region holding in turn the swizzled slab [G][C], the
-// per-warp FFT scratch and the coil images [C][N] | (epi_smem) the epilogue inputs of the
-// row, fetched in the slab's copy group: maps [C][N] (with smaps), p row [N] (mode 2),
-// scaling row [N] float. Without epi_smem the epilogue reads them from global memory.
+// Shared memory: FFT rows [G + R1][C], then the coil images [N][C+1] in their place |
+// (epi_smem) the epilogue inputs of the row, copied while the line is transformed: maps
+// [C][N] (with smaps), p row [N] (modes 2, 3, 5), r or b row [N] (modes 2 with r, 3), scaling
+// row [N] float. Without epi_smem the epilogue reads them from global memory.
 // Mode 2 with r given also writes Re <r, Ap>, <Ap, Ap> and <r, r> per line into
 // parts[lines + i0], parts[2 lines + i0] and parts[3 lines + i0], for the next forward rows to
 // finish the CG update (mode 4 there).
 // Reference: ifft512_rows8_regular_crop_scale (nufft_custom_fft_forward_bench.cu:1517-1552)
 // followed by sense_combine_scaled (nufft_fp16x2_cg_bench.cu:27-54).
-template <int G, int CC>
-__global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ out,
-                                                     int mode, float2* __restrict__ x, float2* __restrict__ r,
-                                                     const float2* __restrict__ p, double* __restrict__ parts,
-                                                     CgState* __restrict__ st, int iter, float inv_scale2,
-                                                     float lambda_scaled, int region, int epi_smem) {
-  constexpr int P = G / 32;
+template <int G, int C>
+__global__ void TSN_ROW_BOUNDS((LineFft<G, C, true>::THREADS))
+inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ out, int mode, float2* __restrict__ x,
+                float2* __restrict__ r, const float2* __restrict__ p, double* __restrict__ parts,
+                CgState* __restrict__ st, int iter, float inv_scale2, float lambda_scaled, int region, int epi_smem) {
+  using F = LineFft<G, C, true>;
   extern __shared__ __align__(16) uint8_t sm[];
   const int N = f.N;
-  constexpr int C = CC;  // coils (one warp each), a compile-time stride
   const int lines = f.lines();
   const int64_t pix_n = f.pix();
-  float2* tw_s = reinterpret_cast<float2*>(sm);
-  uint8_t* reg = reinterpret_cast<uint8_t*>(tw_s + G);
-  float2* emaps = reinterpret_cast<float2*>(reg + region);
+  float2* buf = reinterpret_cast<float2*>(sm);
+  float2* emaps = reinterpret_cast<float2*>(sm + region);
   float2* eprow = emaps + (f.smaps ? C * N : 0);
-  float* escale = reinterpret_cast<float*>(eprow + (mode >= 2 ? N : 0));
+  float2* errow = eprow + (mode >= 2 ? N : 0);
+  const float2* rsrc = mode == 2 ? r : mode == 3 ? x : nullptr;  // r, or the right-hand side b
+  float* escale = reinterpret_cast<float*>(errow + (rsrc ? N : 0));
   __shared__ double red[132];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, c = tid % C;
   // part 1: rows no kernel of a solve writes (coil maps, deapodization); part 2: the rest
   auto issue = [&](int i0, int part) {
     const size_t off = static_cast<size_t>(i0) * N;
-    if (part & 2) {
-      float2* dst = reinterpret_cast<float2*>(reg);
-      // G runs of C complex values (8C bytes each, 16-byte aligned for even C), swizzled
-      const int chn = C / 2;
-      const int k = threadIdx.x % chn;  // 32*C threads: 64 rows per pass
-      for (int q1 = threadIdx.x / chn; q1 < G; q1 += 64)
-        cp_async16(dst + q1 * C + 2 * (k ^ slab_swz(q1, chn)), w1 + (static_cast<size_t>(q1) * lines + i0) * C + 2 * k);
-      if (epi_smem && mode >= 2) cp_async_bytes(eprow, p + off, N * 8);
-    }
     if (epi_smem && (part & 1)) {
       if (f.smaps)
-        for (int c = 0; c < C; ++c) cp_async_bytes(emaps + c * N, f.smaps + static_cast<size_t>(c) * pix_n + off, N * 8);
+        for (int cc = 0; cc < C; ++cc)
+          cp_async_bytes(emaps + cc * N, f.smaps + static_cast<size_t>(cc) * pix_n + off, N * 8);
       cp_async_bytes(escale, f.scaling + off, N * 4);
+    }
+    if (epi_smem && (part & 2)) {
+      if (mode >= 2) cp_async_bytes(eprow, p + off, N * 8);
+      if (rsrc) cp_async_bytes(errow, rsrc + off, N * 8);
     }
     cp_async_commit();
   };
-  cp_async_bytes(tw_s, f.tw, G * 8);
   if (blockIdx.x < lines) issue(blockIdx.x, 1);
   pdl_wait();
   pdl_trigger();
@@ -1067,47 +868,54 @@ __global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_rows_kernel(FftArgs f,
   if (mode == 2) factor = f.gs() / st->sigma[iter] * inv_scale2;
   else if (mode == 3 || mode == 5) factor = f.gs() / st->sigma_x * inv_scale2;
   else factor = inv_scale2 / st->sigma_y;
-  const int c = warp;
-  const int lane_off = 2 * ((c >> 1) ^ slab_swz(lane, C >> 1)) + (c & 1);
   for (int i0 = blockIdx.x; i0 < lines; i0 += gridDim.x) {
     if (i0 != blockIdx.x) {
       __syncthreads();
       issue(i0, 3);
     }
-    cp_async_wait<0>();
+    const float2* src = w1 + static_cast<size_t>(i0) * C + c;
+    F::first(buf, f.tw, tid, [&](int n) { return src[static_cast<size_t>(n) * lines * C]; });
     __syncthreads();
-    const float2* in_s = reinterpret_cast<const float2*>(reg);
-    float2 v[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int n = warp_fft_in_index<G>(j);
-      v[j] = in_s[FftPlan<G>::R == 1 ? n * C + lane_off : slab_idx(n, c, C)];
+    if constexpr (F::R3 > 1) {
+      F::middle(buf, f.tw, tid);
+      __syncthreads();
     }
-    __syncthreads();
-    warp_fft<G, true>(v, reinterpret_cast<float2*>(reg) + c * FftSmem<G>::SCR, tw_s);
-    __syncthreads();
-    float2* img_s = reinterpret_cast<float2*>(reg);  // [C][N]
+    float2 v[F::ITL][F::RL];
+    F::last(buf, tid, [&](int i, int j, int, float2 val) { v[i][j] = val; });
+    cp_async_wait<0>();
+    __syncthreads();  // the FFT rows are read: the region becomes the coil images
+    float2* img_s = buf;  // [N][C+1]
 #pragma unroll
-    for (int m = 0; m < P; ++m) {
-      int i1 = warp_fft_out_index<G>(m) + f.shift;
-      if (i1 >= G) i1 -= G;
-      if (i1 < N) img_s[c * N + i1] = v[m];
+    for (int i = 0; i < F::ITL; ++i) {
+      const int b = F::last_base(tid, i);
+      if (b < 0) continue;
+#pragma unroll
+      for (int j = 0; j < F::RL; ++j) {
+        int i1 = b + F::NL * j + f.shift;
+        if (i1 >= G) i1 -= G;
+        if (i1 < N) img_s[i1 * (C + 1) + c] = v[i][j];
+      }
     }
     __syncthreads();
     double dot = 0.0, dot_r = 0.0, dot_a = 0.0, dot_rr = 0.0;
-    for (int i1 = threadIdx.x; i1 < N; i1 += blockDim.x) {
+    for (int i1 = tid; i1 < N; i1 += blockDim.x) {
       const size_t pix = static_cast<size_t>(i0) * N + i1;
       const float d = (epi_smem ? escale[i1] : f.scaling[pix]) * factor;
+      const float2* img = img_s + i1 * (C + 1);
       if (!f.smaps) {  // coil images out [C][N][N]
-        for (int cc = 0; cc < C; ++cc) out[static_cast<size_t>(cc) * pix_n + pix] = cscale(img_s[cc * N + i1], d);
+#pragma unroll
+        for (int cc = 0; cc < C; ++cc) out[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
         continue;
       }
-      if (mode == 5 && x)  // the coil images before the combine, [C][N][N]
-        for (int cc = 0; cc < C; ++cc) x[static_cast<size_t>(cc) * pix_n + pix] = cscale(img_s[cc * N + i1], d);
+      if (mode == 5 && x) {  // the coil images before the combine, [C][N][N]
+#pragma unroll
+        for (int cc = 0; cc < C; ++cc) x[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
+      }
       float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
       for (int cc = 0; cc < C; ++cc) {
         const float2 s = epi_smem ? emaps[cc * N + i1] : f.smaps[static_cast<size_t>(cc) * pix_n + pix];
-        acc = cadd(acc, cmulc(img_s[cc * N + i1], s));
+        acc = cadd(acc, cmulc(img[cc], s));
       }
       acc = cscale(acc, d);
       if (mode == 0) {
@@ -1124,13 +932,13 @@ __global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_rows_kernel(FftArgs f,
           out[pix] = acc;
           dot += static_cast<double>(pv.x) * acc.x + static_cast<double>(pv.y) * acc.y;
           if (mode == 2 && r) {
-            const float2 rv = r[pix];
+            const float2 rv = epi_smem ? errow[i1] : r[pix];
             dot_r += static_cast<double>(rv.x) * acc.x + static_cast<double>(rv.y) * acc.y;
             dot_a += static_cast<double>(acc.x) * acc.x + static_cast<double>(acc.y) * acc.y;
             dot_rr += static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
           }
         } else {  // reliable residual r = b - M v (b read through x)
-          const float2 bv = x[pix];
+          const float2 bv = epi_smem ? errow[i1] : x[pix];
           const float2 rv = make_float2(bv.x - acc.x, bv.y - acc.y);
           out[pix] = rv;
           dot += static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
@@ -1139,7 +947,7 @@ __global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_rows_kernel(FftArgs f,
     }
     if (mode == 2 && r) {
       const double4 t = block_sum4(dot, dot_r, dot_a, dot_rr, red);
-      if (threadIdx.x == 0) {
+      if (tid == 0) {
         parts[i0] = t.x;
         parts[lines + i0] = t.y;
         parts[2 * static_cast<int64_t>(lines) + i0] = t.z;
@@ -1147,7 +955,7 @@ __global__ void TSN_FFT_BOUNDS(G, (CC <= 8 ? 8 : 16)) inv_rows_kernel(FftArgs f,
       }
     } else if (mode != 0) {
       const double t = block_sum(dot, red);
-      if (threadIdx.x == 0) parts[i0] = t;
+      if (tid == 0) parts[i0] = t;
     }
   }
 }
@@ -1223,49 +1031,16 @@ __global__ void cg_finish_kernel(int nparts, const double* __restrict__ rr_parts
 // ------------------------------------------------------------------------------------------
 // Launchers
 // ------------------------------------------------------------------------------------------
-constexpr size_t kFftTwoCtaSmem = 114 * 1024;  // at most this per CTA keeps two CTAs per SM
-
 static size_t align16(size_t b) { return (b + 15) & ~static_cast<size_t>(15); }
 
-template <int G>
-static size_t fft_scratch_bytes(int C) {
-  return sizeof(float2) * static_cast<size_t>(C) * FftSmem<G>::SCR;
+// Shared memory of the FFT rows of a line of C coils
+template <int G, int C>
+static size_t fft_rows_bytes() {
+  return sizeof(float2) * static_cast<size_t>(LineFft<G, C, false>::ROWS) * C;
 }
-template <int G>
-static size_t fwd_rows_region(const FftArgs& f, int mode) {
-  const size_t in = static_cast<size_t>((mode == 4 ? 4 : 2) + f.C) * f.N * 8 + static_cast<size_t>(f.N) * 4;
-  const size_t out = sizeof(float2) * static_cast<size_t>(G) * (f.C + 1);
-  return align16(std::max({in, out, fft_scratch_bytes<G>(f.C)}));
-}
-template <int G>
-static size_t fwd_cols_region(const FftArgs& f) {
-  const size_t in = sizeof(float2) * static_cast<size_t>(f.N) * f.C;
-  const size_t out = sizeof(uint32_t) * static_cast<size_t>(G) * (2 * f.C + 1);
-  return align16(std::max({in, out, fft_scratch_bytes<G>(f.C)}));
-}
-template <int G>
-static size_t inv_cols_region(const FftArgs& f) {
-  const size_t in = sizeof(float2) * static_cast<size_t>(G) * f.C;
-  const size_t out = sizeof(float2) * static_cast<size_t>(f.N) * (f.C + 1);
-  return align16(std::max({in, out, fft_scratch_bytes<G>(f.C)}));
-}
-// middle stages: [G][C+1] float2 covers the [N][C] / [G][C] slabs and the [N][C+1] output
-template <int G>
-static size_t mid_region(const FftArgs& f) {
-  const size_t rows = sizeof(float2) * static_cast<size_t>(G) * (f.C + 1);
-  return align16(std::max(rows, fft_scratch_bytes<G>(f.C)));
-}
-template <int G>
-static size_t inv_rows_region(const FftArgs& f) {
-  const size_t in = sizeof(float2) * static_cast<size_t>(G) * f.C;
-  const size_t img = sizeof(float2) * static_cast<size_t>(f.C) * f.N;
-  return align16(std::max({in, img, fft_scratch_bytes<G>(f.C)}));
-}
-static size_t inv_rows_epi(const FftArgs& f, int mode) {
-  const size_t maps = f.smaps ? sizeof(float2) * static_cast<size_t>(f.C) * f.N : 0;
-  const size_t prow = mode >= 2 ? sizeof(float2) * static_cast<size_t>(f.N) : 0;
-  return align16(maps + prow + sizeof(float) * static_cast<size_t>(f.N));
-}
+// The row stages stage their coil-map rows (and other epilogue rows) in shared memory while
+// two CTAs still fit on an SM with them; larger lines read them from global memory.
+constexpr size_t kFftStageSmem = 114 * 1024;
 
 template <class K>
 static void ensure_smem(K k, size_t bytes) {
@@ -1283,14 +1058,14 @@ static int sm_count() {
   return n;
 }
 
-// persistent grid: resident CTAs per SM x SMs (a 1/share slice of them when batched cases
-// run side by side), capped by the item count
+// One CTA per item; batched cases (share > 1) run on a 1/share slice of the resident CTAs and
+// loop, so that kernels of other cases run beside them.
 template <class K>
-static int persistent_grid(K k, int threads, size_t smem, int items, int share = 1) {
+static int fft_grid(K k, int threads, size_t smem, int items, int share) {
+  if (share <= 1) return std::max(1, items);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
-  const int grid = std::max(1, std::max(1, per_sm) * sm_count() / std::max(1, share));
-  return std::max(1, std::min(grid, items));
+  return std::max(1, std::min(items, std::max(1, per_sm) * sm_count() / share));
 }
 
 #define TSN_G_SWITCH(G_, ...)                                  \
@@ -1304,7 +1079,7 @@ static int persistent_grid(K k, int threads, size_t smem, int items, int share =
     default: break;                                            \
   }
 // FFT stage instantiation per coil count (4, 8, 12, 16): the index arithmetic folds to
-// constants, and CTAs of up to 8 warps keep three per SM
+// constants
 #define TSN_FFT_C(C_, ...)                                  \
   switch (C_) {                                             \
     case 4: { constexpr int CC = 4; __VA_ARGS__; } break;   \
@@ -1317,60 +1092,48 @@ static int persistent_grid(K k, int threads, size_t smem, int items, int share =
 void launch_fwd_rows(const FftArgs& f, const float2* x, float2* z1, int mode, float2* p, float2* r,
                      const double* partials, int nparts, CgState* st, int iter, cudaStream_t s, float2* xs,
                      const float2* ap) {
-  TSN_G_SWITCH(f.G, {
-    const size_t sm = sizeof(float2) * GG + fwd_rows_region<GG>(f, mode);
-    TSN_FFT_C(f.C, {
-      auto k = fwd_rows_kernel<GG, CC>;
-      ensure_smem(k, sm);
-      const int grid = persistent_grid(k, 32 * f.C, sm, f.lines(), f.share);
-      launch_k(k, grid, 32 * f.C, sm, s, false, f, x, z1, mode, p, r, partials, nparts, st, iter, xs, ap);
-    });
-  });
+  TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
+    const int rows = mode == 4 ? 4 : mode >= 1 ? 2 : 1;
+    const size_t base = fft_rows_bytes<GG, CC>() + (sizeof(float2) * rows + sizeof(float)) * static_cast<size_t>(f.N);
+    const size_t maps = sizeof(float2) * static_cast<size_t>(CC) * map_pitch(f.N);
+    const int stage = f.smaps && base + maps <= kFftStageSmem ? 1 : 0;
+    const size_t sm = base + (stage ? maps : 0);
+    constexpr int T = LineFft<GG, CC, false>::THREADS;
+    auto k = fwd_rows_kernel<GG, CC>;
+    ensure_smem(k, sm);
+    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, false, f, x, z1, mode, p, r, partials, nparts, st,
+             iter, xs, ap, stage);
+  }));
 }
 
 void launch_fwd_cols(const FftArgs& f, const float2* z1, __half* panel, cudaStream_t s) {
-  TSN_G_SWITCH(f.G, {
-    const size_t region = fwd_cols_region<GG>(f);
-    const size_t base = sizeof(float2) * GG;
-    const int nbuf = base + 2 * region <= kFftTwoCtaSmem ? 2 : 1;
-    const size_t sm = base + nbuf * region;
-    TSN_FFT_C(f.C, {
-      auto k = fwd_cols_kernel<GG, CC>;
-      ensure_smem(k, sm);
-      const int grid = persistent_grid(k, 32 * f.C, sm, f.gcols(), f.share);
-      launch_k(k, grid, 32 * f.C, sm, s, false, f, z1, panel, static_cast<int>(region), nbuf);
-    });
-  });
+  TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
+    constexpr int W = cols_coils(CC), T = LineFft<GG, W, false>::THREADS;
+    const size_t sm = fft_rows_bytes<GG, W>();
+    auto k = fwd_cols_kernel<GG, CC>;
+    ensure_smem(k, sm);
+    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, false, f, z1, panel);
+  }));
 }
 
 void launch_fwd_mid(const FftArgs& f, const float2* z1, float2* z2, cudaStream_t s) {
-  TSN_G_SWITCH(f.G, {
-    const size_t region = mid_region<GG>(f);
-    const size_t base = sizeof(float2) * GG;
-    const int nbuf = base + 2 * region <= kFftTwoCtaSmem ? 2 : 1;
-    const size_t sm = base + nbuf * region;
-    TSN_FFT_C(f.C, {
-      auto k = fwd_mid_kernel<GG, CC>;
-      ensure_smem(k, sm);
-      const int grid = persistent_grid(k, 32 * f.C, sm, f.N * f.G, f.share);
-      launch_k(k, grid, 32 * f.C, sm, s, false, f, z1, z2, static_cast<int>(region), nbuf);
-    });
-  });
+  TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
+    constexpr int W = cols_coils(CC), T = LineFft<GG, W, false>::THREADS;
+    const size_t sm = fft_rows_bytes<GG, W>();
+    auto k = fwd_mid_kernel<GG, CC>;
+    ensure_smem(k, sm);
+    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, false, f, z1, z2);
+  }));
 }
 
 void launch_inv_mid(const FftArgs& f, const float2* z2, float2* z1, cudaStream_t s) {
-  TSN_G_SWITCH(f.G, {
-    const size_t region = mid_region<GG>(f);
-    const size_t base = sizeof(float2) * GG;
-    const int nbuf = base + 2 * region <= kFftTwoCtaSmem ? 2 : 1;
-    const size_t sm = base + nbuf * region;
-    TSN_FFT_C(f.C, {
-      auto k = inv_mid_kernel<GG, CC>;
-      ensure_smem(k, sm);
-      const int grid = persistent_grid(k, 32 * f.C, sm, f.N * f.G, f.share);
-      launch_k(k, grid, 32 * f.C, sm, s, false, f, z2, z1, static_cast<int>(region), nbuf);
-    });
-  });
+  TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
+    constexpr int W = cols_coils(CC), T = LineFft<GG, W, true>::THREADS;
+    const size_t sm = fft_rows_bytes<GG, W>();
+    auto k = inv_mid_kernel<GG, CC>;
+    ensure_smem(k, sm);
+    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, false, f, z2, z1);
+  }));
 }
 
 void launch_split_samples(const float2* y, const float* density, int64_t m, int c, __half* panel,
@@ -1381,36 +1144,30 @@ void launch_split_samples(const float2* y, const float* density, int64_t m, int 
 }
 
 void launch_inv_cols(const FftArgs& f, const float2* grid, float2* w1, cudaStream_t s) {
-  TSN_G_SWITCH(f.G, {
-    const size_t region = inv_cols_region<GG>(f);
-    const size_t base = sizeof(float2) * GG;
-    const int nbuf = base + 2 * region <= kFftTwoCtaSmem ? 2 : 1;
-    const size_t sm = base + nbuf * region;
-    TSN_FFT_C(f.C, {
-      auto k = inv_cols_kernel<GG, CC>;
-      ensure_smem(k, sm);
-      const int g = persistent_grid(k, 32 * f.C, sm, f.gcols(), f.share);
-      launch_k(k, g, 32 * f.C, sm, s, false, f, grid, w1, static_cast<int>(region), nbuf);
-    });
-  });
+  TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
+    constexpr int W = cols_coils(CC), T = LineFft<GG, W, true>::THREADS;
+    const size_t sm = fft_rows_bytes<GG, W>();
+    auto k = inv_cols_kernel<GG, CC>;
+    ensure_smem(k, sm);
+    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, false, f, grid, w1);
+  }));
 }
 
 void launch_inv_rows(const FftArgs& f, const float2* w1, float2* out, int mode, float2* x, float2* r, const float2* p,
                      double* partials, CgState* st, int iter, float inv_scale2, float lambda_scaled, cudaStream_t s) {
-  TSN_G_SWITCH(f.G, {
-    const size_t region = inv_rows_region<GG>(f);
-    const size_t base = sizeof(float2) * GG + region;
-    const size_t epi = inv_rows_epi(f, mode);
-    const int epi_smem = base + epi <= kFftTwoCtaSmem ? 1 : 0;
-    const size_t sm = base + (epi_smem ? epi : 0);
-    TSN_FFT_C(f.C, {
-      auto k = inv_rows_kernel<GG, CC>;
-      ensure_smem(k, sm);
-      const int g = persistent_grid(k, 32 * f.C, sm, f.lines(), f.share);
-      launch_k(k, g, 32 * f.C, sm, s, false, f, w1, out, mode, x, r, p, partials, st, iter, inv_scale2, lambda_scaled,
-                 static_cast<int>(region), epi_smem);
-    });
-  });
+  TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
+    const size_t img = sizeof(float2) * static_cast<size_t>(f.N) * (CC + 1);
+    const size_t region = align16(std::max(fft_rows_bytes<GG, CC>(), img));
+    const int rows = (f.smaps ? CC : 0) + (mode >= 2 ? 1 : 0) + ((mode == 2 && r) || mode == 3 ? 1 : 0);
+    const size_t epi = (sizeof(float2) * rows + sizeof(float)) * static_cast<size_t>(f.N);
+    const int epi_smem = region + epi <= kFftStageSmem ? 1 : 0;
+    const size_t sm = region + (epi_smem ? epi : 0);
+    constexpr int T = LineFft<GG, CC, true>::THREADS;
+    auto k = inv_rows_kernel<GG, CC>;
+    ensure_smem(k, sm);
+    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, false, f, w1, out, mode, x, r, p, partials, st, iter,
+             inv_scale2, lambda_scaled, static_cast<int>(region), epi_smem);
+  }));
 }
 
 void launch_cg_update(int N, int lines, int nparts, float2* x, float2* r, const float2* p, const float2* ap,

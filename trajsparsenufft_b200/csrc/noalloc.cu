@@ -97,7 +97,6 @@ DeviceSetup& setup_device(int device, cudaStream_t s) {
     }
     if ((e = cudaMemcpyToSymbol(g_static_twiddle, tw.data(), sizeof(float2) * tw.size())) != cudaSuccess)
       cuda_fail(e, "twiddle init");
-    tsn::set_twiddle_constants(s);
     d.scratch = static_cast<float2*>(p_scratch);
   }
   return d;

@@ -103,10 +103,6 @@ struct GraphKey {
   }
 };
 
-// __constant__ twiddle tables are per device: filled once for each device a plan lives on
-std::mutex g_const_mutex;
-std::vector<int> g_const_devices;
-
 }  // namespace
 
 struct tsn_plan {
@@ -578,15 +574,6 @@ void allocate_workspaces(tsn_plan* P) {
   P->info.dims = P->dims;
   P->info.workspace_bytes = static_cast<int64_t>(P->z1.bytes + P->z2.bytes + P->panel.bytes + P->spanel.bytes +
                                                  P->grid.bytes + 4 * P->r.bytes + P->state.bytes);
-  {
-    std::lock_guard<std::mutex> lock(g_const_mutex);
-    int dev = 0;
-    CUDA_OK(cudaGetDevice(&dev));
-    if (std::find(g_const_devices.begin(), g_const_devices.end(), dev) == g_const_devices.end()) {
-      set_twiddle_constants(nullptr);
-      g_const_devices.push_back(dev);
-    }
-  }
   CUDA_OK(cudaGetLastError());
 }
 
