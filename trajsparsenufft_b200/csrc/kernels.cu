@@ -581,7 +581,6 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
   } else {
     total = sum_partials(parts, nparts, red);
   }
-  const float af = static_cast<float>(alpha);
   float sigma;
   double beta = 0.0;
   if (mode == 0) {
@@ -598,7 +597,6 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
       st->sigma[iter] = sigma;
     }
   }
-  const float bf = static_cast<float>(beta);
   const float scl = sigma / f.gs();
   const bool sense = f.smaps || mode >= 1;
   for (int i0 = blockIdx.x; i0 < lines; i0 += gridDim.x) {
@@ -619,13 +617,11 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
       if (has_beta) {
         const float2 pv = row1[i];
         if (mode == 4) {  // x += alpha p, r -= alpha Ap (the previous iteration's update)
-          const float2 av = row2[i], xv = row3[i];
-          v.x -= af * av.x;
-          v.y -= af * av.y;
+          v = axpy64(-alpha, row2[i], v);
           r[off + i] = v;
-          xs[off + i] = make_float2(xv.x + af * pv.x, xv.y + af * pv.y);
+          xs[off + i] = axpy64(alpha, pv, row3[i]);
         }
-        v = make_float2(v.x + bf * pv.x, v.y + bf * pv.y);
+        v = axpy64(beta, pv, v);
       }
       if (mode >= 1) p[off + i] = v;
       row0[i] = cscale(v, d);
@@ -996,17 +992,14 @@ __global__ void cg_update_kernel(int N, int nparts, int lines, float2* __restric
     if (!isfinite(pap)) st->finite_ok = 0;
     if (prior_ok && ok) st->completed = iter + 1;
   }
-  const float af = static_cast<float>(alpha);
   double acc = 0.0;
 #pragma unroll
   for (int j = 0; j < kCgRowPix; ++j) {
     const int i1 = threadIdx.x + j * blockDim.x;
     if (i1 >= N) continue;
     const size_t pix = static_cast<size_t>(i0) * N + i1;
-    xv[j].x += af * pv[j].x;
-    xv[j].y += af * pv[j].y;
-    rv[j].x -= af * av[j].x;
-    rv[j].y -= af * av[j].y;
+    xv[j] = axpy64(alpha, pv[j], xv[j]);
+    rv[j] = axpy64(-alpha, av[j], rv[j]);
     x[pix] = xv[j];
     r[pix] = rv[j];
     acc += static_cast<double>(rv[j].x) * rv[j].x + static_cast<double>(rv[j].y) * rv[j].y;
@@ -1264,6 +1257,12 @@ __global__ void cgb_dots_kernel(int64_t n, const float2* __restrict__ rb, const 
   }
 }
 
+// a x + b y (+ c z) in FP64, one rounding per component
+__device__ __forceinline__ float2 lincomb64(double a, float2 x, double b, float2 y, double c = 0.0,
+                                            float2 z = make_float2(0.f, 0.f)) {
+  return make_float2(static_cast<float>(a * x.x + b * y.x + c * z.x), static_cast<float>(a * x.y + b * y.y + c * z.y));
+}
+
 // sc (device FP64): [0] rho, [1] rho', [2] gamma, [3] rhob in; [4] rhob of step k out.
 __global__ void cgb_update_kernel(int64_t n, int nparts, const double* __restrict__ parts,
                                   const double* __restrict__ rho_p, const double* __restrict__ rhon_p,
@@ -1291,18 +1290,17 @@ __global__ void cgb_update_kernel(int64_t n, int nparts, const double* __restric
   const double alphab = d5 - rb2q;
   const double gammab = -alphab * rho / (gamma * gamma);
   if (blockIdx.x == 0 && threadIdx.x == 0) *rhob_out = -betab * rho_n / (rho * rho) + alphab / gamma;
-  const float a = static_cast<float>(alpha), b = static_cast<float>(beta), g = static_cast<float>(gammab),
-              h = static_cast<float>(2.0 * rhob_n);
+  const double h = 2.0 * rhob_n;
   double acc = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float2 vrb = rb[i], vpb = pb[i], vp = p[i], vq = q[i], vrn = rn[i], vxb = xb[i];
-    const float2 r2 = make_float2(vrb.x + vpb.x + h * vrn.x, vrb.y + vpb.y + h * vrn.y);
+    const float2 r2 = axpy64(h, vrn, make_float2(vrb.x + vpb.x, vrb.y + vpb.y));
     rb[i] = r2;
-    const float2 qv = make_float2(-a * r2.x + g * vp.x, -a * r2.y + g * vp.y);
+    const float2 qv = lincomb64(-alpha, r2, gammab, vp);
     qb[i] = qv;
     acc += static_cast<double>(qv.x) * qv.x + static_cast<double>(qv.y) * qv.y;
-    pb[i] = make_float2(b * vpb.x + a * vxb.x + g * vq.x, b * vpb.y + a * vxb.y + g * vq.y);
+    pb[i] = lincomb64(beta, vpb, alpha, vxb, gammab, vq);
   }
   if (qnorm_parts) {  // |qb|^2 partials: the panel scale of the M qb that follows
     const double t = block_sum(acc, red);
@@ -1344,16 +1342,16 @@ __global__ void cgf_update_kernel(int64_t n, const double* __restrict__ rho_p, c
                                   const float2* __restrict__ r, const float2* __restrict__ q,
                                   float2* __restrict__ x_out, float2* __restrict__ r_out, double* __restrict__ parts) {
   __shared__ double red[33];
-  const float a = static_cast<float>(*rho_p / *gamma_p);
+  const double a = *rho_p / *gamma_p;
   double acc = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float2 vp = p[i], vr = r[i], vq = q[i];
     if (x) {
       const float2 vx = x[i];
-      x_out[i] = make_float2(vx.x + a * vp.x, vx.y + a * vp.y);
+      x_out[i] = axpy64(a, vp, vx);
     }
-    const float2 rn = make_float2(vr.x - a * vq.x, vr.y - a * vq.y);
+    const float2 rn = axpy64(-a, vq, vr);
     r_out[i] = rn;
     acc += static_cast<double>(rn.x) * rn.x + static_cast<double>(rn.y) * rn.y;
   }
@@ -1370,12 +1368,12 @@ __global__ void cgf_direction_kernel(int64_t n, int nparts, const double* __rest
   __shared__ double red[33];
   const double rho_n = sum_partials(parts, nparts, red);
   if (blockIdx.x == 0 && threadIdx.x == 0) *rho_out = rho_n;
-  const float b = static_cast<float>(rho_n / *rho_p);
+  const double b = rho_n / *rho_p;
   double acc = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float2 vp = p[i], vr = r_new[i];
-    const float2 pn = make_float2(vr.x + b * vp.x, vr.y + b * vp.y);
+    const float2 pn = axpy64(b, vp, vr);
     p_out[i] = pn;
     acc += static_cast<double>(pn.x) * pn.x + static_cast<double>(pn.y) * pn.y;
   }
