@@ -62,3 +62,30 @@ def test_adjoint_endpoint_matches_numpy_ifft(name, layout):
     img = full[:, pos[:, None], pos[None, :]] * d[None]
     assert rel_l2(coils, img) <= 2e-5
     assert rel_l2(got, np.sum(np.conj(s) * img, axis=0)) <= 2e-5
+
+
+# Line FFTs at every radix plan (two passes: 128, 256; three: 384, 512, 640, 1024) and coil
+# grouping (16 coils: two CTAs), with image sizes beside half the grid, full grids, and image
+# rows too long for the row stages' shared-memory staging.
+@pytest.mark.parametrize("n,g,c", [(60, 128, 16), (128, 128, 4), (100, 256, 12), (256, 256, 8), (188, 384, 16),
+                                   (260, 512, 4), (512, 512, 16), (300, 640, 8), (412, 1024, 4), (512, 1024, 12)])
+def test_line_fft_endpoints_at_ragged_sizes(n, g, c):
+    from trajsparsenufft_b200 import synth
+    from trajsparsenufft_b200.operator import Plan
+    plan = Plan.from_trajectory(synth.golden_radial(4, 32), im_size=n, grid_size=g, coils=c, width=4)
+    rng = np.random.default_rng(n)
+    cplx = lambda *sh: (rng.standard_normal(sh) + 1j * rng.standard_normal(sh)).astype(np.complex64)
+    x, s, grid = cplx(n, n), cplx(c, n, n), cplx(c, g, g)
+    d, shift = okb.deapodization(n, g, 4), n // 2
+    panel, scale = plan.fft_forward_panel(torch.from_numpy(x).cuda(), torch.from_numpy(s).cuda())
+    p = panel.float().cpu().numpy().astype(np.float64)
+    v = (p[:, : 2 * c] + p[:, 2 * c:]).reshape(g, g, c, 2)
+    got = (v[..., 0] + 1j * v[..., 1]).transpose(2, 1, 0) / scale
+    assert rel_l2(got, np.fft.fft2(_grid_from_image(x[None].astype(np.complex128) * s * d[None], g, shift))) <= 1e-5
+    internal = torch.from_numpy(np.ascontiguousarray(grid.transpose(2, 1, 0).reshape(g * g, c))).cuda()
+    full = np.fft.ifft2(grid.astype(np.complex128)) * g * g
+    pos = (np.arange(n) - shift) % g
+    img = full[:, pos[:, None], pos[None, :]] * d[None]
+    assert rel_l2(plan.fft_adjoint_image(internal).cpu().numpy(), img) <= 2e-5
+    assert rel_l2(plan.fft_adjoint_image(internal, torch.from_numpy(s).cuda()).cpu().numpy(),
+                  np.sum(np.conj(s) * img, axis=0)) <= 2e-5

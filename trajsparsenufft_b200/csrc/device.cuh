@@ -58,18 +58,14 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem_dst)), "l"(gmem_src));
 }
-// 16-byte copy when `live`, else a 16-byte zero store to the same shared address (no global
-// read); predicated, so a warp with mixed lanes does not branch.
-__device__ __forceinline__ void cp_async16_or_zero(void* smem_dst, const void* gmem_src, bool live) {
-  asm volatile(
-      "{\n"
-      "  .reg .pred p;\n"
-      "  setp.ne.b32 p, %2, 0;\n"
-      "  @p cp.async.cg.shared.global [%0], [%1], 16;\n"
-      "  @!p st.shared.v4.u32 [%0], {%3, %3, %3, %3};\n"
-      "}\n" ::"r"(smem_u32(smem_dst)),
-      "l"(gmem_src), "r"(static_cast<int>(live)), "r"(0)
-      : "memory");
+// The same to a shared address.
+__device__ __forceinline__ void cp_async16_u32(uint32_t smem_dst, const void* gmem_src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_dst), "l"(gmem_src) : "memory");
+}
+// 16-byte copy to a shared address (bytes = 16), or a 16-byte zero fill without a global read
+// (bytes = 0).
+__device__ __forceinline__ void cp_async16_zfill(uint32_t smem_dst, const void* gmem_src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_dst), "l"(gmem_src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -77,18 +73,12 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// Four 8x8 b16 matrices (rows addressed by lanes 0-7, 8-15, 16-23, 24-31).
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem_row) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem_row)));
-}
-
 // Four transposed 8x8 b16 matrices (rows addressed by lanes 0-7, 8-15, 16-23, 24-31).
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_row) {
+__device__ __forceinline__ void ldmatrix_x4_trans_u32(uint32_t (&r)[4], uint32_t smem_row) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem_row)));
+               : "r"(smem_row)
+               : "memory");
 }
 
 // Warp-level 2:4 sparse MMA m16n8k32, FP16 inputs, FP32 accumulate, metadata selector 0.
@@ -99,6 +89,16 @@ __device__ __forceinline__ void mma_sp_16832(float (&d)[4], const uint32_t (&a)[
       "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9,%10,%11}, {%0,%1,%2,%3}, %12, 0x0;\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(meta));
+}
+
+// The same product from a zero accumulator.
+__device__ __forceinline__ void mma_sp_16832_zero(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[4],
+                                                  uint32_t meta) {
+  asm volatile(
+      "mma.sp::ordered_metadata.sync.aligned.m16n8k32.row.col.f32.f16.f16.f32 "
+      "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9,%10,%11}, {%13,%13,%13,%13}, %12, 0x0;\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(meta), "f"(0.f));
 }
 
 // FP32 value -> FP16 high part + FP16 residual (value - float(high)), the reference's

@@ -66,7 +66,7 @@ static void launch_k(void (*kernel)(KArgs...), int grid, int block, size_t smem,
 // Sparse interpolation: one warp per 16-row group, 2:4 tiles through mma.sp m16n8k32.
 // Per tile the 32 gathered panel rows (hi and res together) are brought to shared memory
 // with 16-byte cp.async through a per-warp ring, swizzled so ldmatrix.trans is
-// conflict-free; dead (padding) columns are zero-stored and never read.
+// conflict-free; dead (padding) columns are zero-filled and never read.
 // Reference: nufft_gt_spmma_complex_fused_f16_f32 (nufft_spmma_bench.cu:402-663), which
 // gathers B with 2-byte loads and reduces 4 warps through shared memory.
 // ------------------------------------------------------------------------------------------
@@ -91,18 +91,22 @@ __device__ __forceinline__ int32_t record_row(const uint8_t* rows24, int32_t fla
   return ((static_cast<uint32_t>(flags) >> (kRecLiveShift + s)) & 1u) ? static_cast<int32_t>(v) : -1;
 }
 
-// Per-warp shared-memory ring: stage = tile record (cols, A, meta) + 32 gathered panel rows.
-// Records are fetched kRecAhead tiles ahead, gathers kGatherAhead tiles ahead (the gather
-// needs the record's column ids), so a warp waits only on cp.async groups, never on a
-// register load.  Warps are persistent: each streams a contiguous, tile-balanced run of
-// work items and the pipeline runs across item boundaries.  The ring depth STAGES is per
-// view (InterpView::stages): three stages (34 KB per 4-warp CTA, 24 warps per SM) when the
-// gathered panel sits in L2, which measured faster than deeper rings with fewer warps;
-// four stages (45 KB, 20 warps per SM, records one tile further ahead) when it does not and
-// gathers wait on DRAM (3D grids: 1.33 vs 1.79 ms per forward launch).  Records run
-// STAGES - 1 tiles ahead, gathers kGatherAhead.
-constexpr int kGatherAhead = 1;
-
+// Per-warp shared-memory rings: kRingRecords tile records (offsets, A, meta, rows) and
+// kRingGathers stages of 32 gathered panel rows. Records are fetched three tiles ahead,
+// gathers one (the gather needs the record's offsets), so a warp waits only on cp.async
+// groups, never on a register load.  Warps are persistent: each streams a contiguous,
+// tile-balanced run of work items and the pipeline runs across item boundaries.
+// Measured on 10-iteration solves (us): four records 594 / 1009 (256^2 with 8 / 16 coils)
+// against three records 625 / 1016, three gather stages 625 / 1209 (fewer warps fit), and
+// everything but the gathered rows in registers instead of shared memory 615 / 1112.
+constexpr int kRingRecords = 4, kRingGathers = 2;
+__host__ __device__ constexpr int interp_smem(int rowh, int ncomp) {
+  return kInterpWarps * (kRingRecords * record_bytes(ncomp) + kRingGathers * 32 * rowh * 2);
+}
+// CTAs that an SM's shared memory (228 KB, 1 KB reserved per CTA) holds; registers follow
+__host__ __device__ constexpr int interp_ctas(int rowh, int ncomp) {
+  return 228 * 1024 / (interp_smem(rowh, ncomp) + 1024) < 10 ? 228 * 1024 / (interp_smem(rowh, ncomp) + 1024) : 10;
+}
 // Writes one finished item: split chunks publish their accumulators and the last chunk of
 // the group reduces all chunks in chunk order; whole groups and finishing chunks apply the
 // epilogue.
@@ -114,13 +118,14 @@ __device__ __forceinline__ void interp_finish_item(float (&acc)[NCOMP][NA][4], c
   if (info.split >= 0) {
     const int split = info.split;
     const int chunk = info.chunk & 0xFFFF, nchunks = info.chunk >> 16;
-    float* mine = v.partials + static_cast<size_t>(info.first_slot + chunk) * kPartialFloats * 32;
+    // partial sums [chunk slot][component][coil block][lane] float4
+    float4* slots = reinterpret_cast<float4*>(v.partials) + static_cast<size_t>(info.first_slot) * kPartialFloats * 8 + lane;
+    float4* mine = slots + chunk * kPartialFloats * 8;
 #pragma unroll
     for (int c = 0; c < NCOMP; ++c)
 #pragma unroll
       for (int a2 = 0; a2 < NA; ++a2)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) mine[((c * NA + a2) * 4 + i) * 32 + lane] = acc[c][a2][i];
+        mine[(c * NA + a2) * 32] = make_float4(acc[c][a2][0], acc[c][a2][1], acc[c][a2][2], acc[c][a2][3]);
     __threadfence();
     __syncwarp();
     int prior = 0;
@@ -128,21 +133,33 @@ __device__ __forceinline__ void interp_finish_item(float (&acc)[NCOMP][NA][4], c
     prior = __shfl_sync(0xFFFFFFFFu, prior, 0);
     if (prior != nchunks - 1) return;
     __threadfence();
+    // The last chunk to arrive is the launch's critical path (a central grid cell has tens of
+    // chunks): kBatch loads travel together, the sums stay in chunk order.
+    constexpr int kBatch = 8;
 #pragma unroll
     for (int c = 0; c < NCOMP; ++c)
 #pragma unroll
-      for (int a2 = 0; a2 < NA; ++a2)
+      for (int a2 = 0; a2 < NA; ++a2) {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4* src = slots + (c * NA + a2) * 32;
+        for (int k0 = 0; k0 < nchunks; k0 += kBatch) {
+          float4 t[kBatch];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[c][a2][i] = 0.f;
-    for (int k = 0; k < nchunks; ++k) {
-      const float* src = v.partials + static_cast<size_t>(info.first_slot + k) * kPartialFloats * 32;
+          for (int k = 0; k < kBatch; ++k)
+            t[k] = k0 + k < nchunks ? __ldcg(src + (k0 + k) * kPartialFloats * 8) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int c = 0; c < NCOMP; ++c)
-#pragma unroll
-        for (int a2 = 0; a2 < NA; ++a2)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[c][a2][i] += __ldcg(src + ((c * NA + a2) * 4 + i) * 32 + lane);
-    }
+          for (int k = 0; k < kBatch; ++k) {
+            sum.x += t[k].x;
+            sum.y += t[k].y;
+            sum.z += t[k].z;
+            sum.w += t[k].w;
+          }
+        }
+        acc[c][a2][0] = sum.x;
+        acc[c][a2][1] = sum.y;
+        acc[c][a2][2] = sum.z;
+        acc[c][a2][3] = sum.w;
+      }
     if (lane == 0) v.counters[split] = 0;  // ready for the next launch
   }
   if constexpr (EPI == EPI_RAW) {
@@ -197,32 +214,39 @@ __device__ __forceinline__ void interp_finish_item(float (&acc)[NCOMP][NA][4], c
   }
 }
 
-template <int ROWH, bool SPLIT, int NCOMP, int EPI, bool CONJ, int STAGES, bool SUMC = false>
-__global__ void __launch_bounds__(kInterpWarps * 32) interp_mmasp_kernel(InterpView v, const __half* __restrict__ panel,
+//
+// What bounds it: instruction issue and the latency of the chain record -> gather -> MMA; with
+// both data streams left out a launch still takes three quarters of its time. So the record
+// holds what a lane needs as the lane needs it (the byte offsets of its gathers in one shared
+// load, A as MMA fragments) instead of column ids that were passed around by shuffles and
+// tested for every 16-byte copy (209 warp instructions per tile). 10-iteration solves: 256^2
+// with 8 coils 615 -> 594 us, with 16 coils 1210 -> 1009 us, 128^2 with 4 coils 343 -> 322 us.
+template <int ROWH, bool SPLIT, int NCOMP, int EPI, bool CONJ, bool SUMC = false>
+__global__ void __launch_bounds__(kInterpWarps * 32, interp_ctas(ROWH, NCOMP)) interp_mmasp_kernel(InterpView v, const __half* __restrict__ panel,
                                                                          InterpOut o) {
-  constexpr int kStages = STAGES;
-  constexpr int kRecAhead = STAGES - 1;
+  constexpr int NR = kRingRecords, NG = kRingGathers;
+  constexpr int kRecAhead = NR - 1, kGatherAhead = NG - 1;
   constexpr int BYTES = ROWH * 2;
   constexpr int CH = BYTES / 16;
+  constexpr int LPR = gather_lanes(ROWH);  // lanes sharing a row
+  constexpr int NOFF = LPR;                // rows per lane: 32 / (32 / LPR)
+  constexpr int NSUB = CH / LPR;           // chunks of each row per lane
   constexpr int NB = ROWH / 8;
   constexpr int NA = SPLIT ? NB / 2 : NB;
   constexpr int NACC = NCOMP * NA * 4;
   constexpr int INFO = 128 + 576 * NCOMP;         // RecordInfo offset in the record
   constexpr int REC = record_bytes(NCOMP);        // record bytes (all staged)
-  constexpr int STAGE = REC + 32 * BYTES;
-  constexpr unsigned FULL = 0xFFFFFFFFu;
+  constexpr int STAGE = 32 * BYTES;
   static_assert(NACC <= kPartialFloats, "partials slot too small");
-  static_assert(REC % 16 == 0 && STAGE % 16 == 0, "16-byte stages");
-  static_assert(kGatherAhead >= 1 && kRecAhead > kGatherAhead && kStages == kRecAhead + 1, "ring arithmetic");
+  static_assert(REC % 16 == 0 && STAGE % 128 == 0, "16-byte records, aligned stages");
+  static_assert(kGatherAhead >= 1 && kRecAhead > kGatherAhead, "ring arithmetic");
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wid = blockIdx.x * kInterpWarps + warp;
   if (wid >= v.n_warps) return;
   const int2 range = v.warp_ranges[wid];
   const int n = range.y - range.x;
-  const uint8_t* recs = v.records + static_cast<size_t>(range.x) * REC;
-  uint8_t* ring = smem + warp * kStages * STAGE;
-  const uint8_t* pb = reinterpret_cast<const uint8_t*>(panel);
+  const uint8_t* rec_src = v.records + static_cast<size_t>(range.x) * REC + 16 * lane;
   const int g = lane >> 2;
   float scale = o.scale_mul;
   // records are plan data: their first copies stream in while the preceding kernel drains;
@@ -248,43 +272,65 @@ __global__ void __launch_bounds__(kInterpWarps * 32) interp_mmasp_kernel(InterpV
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[c][a][i] = 0.f;
 
-  // Per-lane gather constants: chunk i of this lane is 16-byte chunk (lane + 32 i) % CH of
-  // gathered row (lane + 32 i) / CH; its swizzled shared offset and source byte offset.
-  int g_row[CH];
-  uint32_t g_dst[CH], g_src[CH];
-#pragma unroll
-  for (int i = 0; i < CH; ++i) {
-    const int ci = lane + 32 * i;
-    const int row = ci / CH, ch = ci % CH;
-    g_row[i] = row;
-    g_dst[i] = static_cast<uint32_t>(REC + row * BYTES + chunk_swizzle<CH>(ch, row) * 16);
-    g_src[i] = static_cast<uint32_t>(ch * 16);
-  }
-  // k-th record of this warp -> ring stage st
-  auto issue_record = [&](int k, uint8_t* st) {
+  // gather stages of all warps first (128-byte aligned), then the records
+  const uint8_t* rec_ring = smem + kInterpWarps * NG * STAGE + warp * NR * REC;
+  const uint32_t gat_ring = smem_u32(smem + warp * NG * STAGE);
+  // This lane's source chunk and its swizzled place in stage 0: row i of a lane lies
+  // i * (32 / LPR) rows further with the same swizzle, but for 128-byte rows, where odd rows
+  // flip chunk bit 2.
+  const uint8_t* pb = reinterpret_cast<const uint8_t*>(panel) + (lane % LPR) * 16;
+  const uint32_t dst0 =
+      gat_ring + static_cast<uint32_t>((lane / LPR) * BYTES + chunk_swizzle<CH>(lane % LPR, lane / LPR) * 16);
+  // this lane's ldmatrix row in stage 0; chunk nb flips address bits (the stages are aligned)
+  const uint32_t ldm0 = gat_ring + static_cast<uint32_t>(lane * BYTES + chunk_swizzle<CH>(0, lane) * 16);
+  auto ldm = [&](int nb) {
+    return CH == 6 ? gat_ring + static_cast<uint32_t>(lane * BYTES + chunk_swizzle<CH>(nb, lane) * 16) : ldm0 ^ (nb * 16u);
+  };
+  // k-th record of this warp -> its ring slot
+  auto issue_record = [&](int k, int slot) {
     if (k < n) {
-      const uint8_t* src = recs + static_cast<size_t>(k) * REC;
+      const uint32_t dst = smem_u32(rec_ring) + slot * REC + 16 * lane;
 #pragma unroll
       for (int c0 = 0; c0 < REC / 16; c0 += 32)
-        if (c0 + 32 <= REC / 16 || lane < REC / 16 - c0) cp_async16(st + 16 * (c0 + lane), src + 16 * (c0 + lane));
+        if (c0 + 32 <= REC / 16 || lane < REC / 16 - c0) cp_async16_u32(dst + 16 * c0, rec_src + 16 * c0);
+      rec_src += REC;
     }
     cp_async_commit();  // empty groups keep the group arithmetic uniform
   };
-  auto issue_gather = [&](int k, uint8_t* st) {
+  auto issue_gather = [&](int k, int slot, int stage) {
     if (k >= 0 && k < n) {
       wait_dep();
-      const int32_t col = reinterpret_cast<const int32_t*>(st)[lane];
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(rec_ring + slot * REC) + (lane / LPR) * NOFF;
+      uint32_t f[NOFF];
+      if constexpr (NOFF == 2) {
+        const uint2 t = *reinterpret_cast<const uint2*>(q);
+        f[0] = t.x;
+        f[1] = t.y;
+      } else {
 #pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int src = __shfl_sync(FULL, col, g_row[i]);
-        cp_async16_or_zero(st + g_dst[i], pb + static_cast<size_t>(static_cast<uint32_t>(max(src, 0)) * BYTES) + g_src[i],
-                           src >= 0);
+        for (int i = 0; i < NOFF; i += 4) {
+          const uint4 t = *reinterpret_cast<const uint4*>(q + i);
+          f[i] = t.x;
+          f[i + 1] = t.y;
+          f[i + 2] = t.z;
+          f[i + 3] = t.w;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NOFF; ++i) {
+        const uint32_t bytes = ~f[i] & kGatherDead;  // 16, or 0 (zero fill, no read) for a dead column
+        const uint8_t* src = pb + f[i];
+#pragma unroll
+        for (int u = 0; u < NSUB; ++u)
+          cp_async16_zfill((CH == 8 && (i & 1) ? dst0 ^ 64u : dst0) + stage * STAGE + i * (32 / LPR) * BYTES + u * LPR * 16,
+                           src + u * LPR * 16, bytes);
       }
     }
     cp_async_commit();
   };
-  auto compute = [&](uint8_t* st) {
+  auto compute = [&](int slot, int stage) {
     wait_dep();
+    const uint8_t* st = rec_ring + slot * REC;
     const RecordInfo info = *reinterpret_cast<const RecordInfo*>(st + INFO);
     const uint8_t* trow = st + INFO + 16;
     if constexpr (EPI == EPI_PANEL) {  // density weights at the item's first tile
@@ -297,27 +343,40 @@ __global__ void __launch_bounds__(kInterpWarps * 32) interp_mmasp_kernel(InterpV
     uint32_t a[NCOMP][4], meta[NCOMP];
 #pragma unroll
     for (int c = 0; c < NCOMP; ++c) {
-      // A rows of 32 B; the 16-B halves of row r are stored swapped when (r >> 2) & 1
-      const int r = (lane & 7) + ((lane >> 3) & 1) * 8;
-      const int half = lane >> 4;
-      ldmatrix_x4(a[c], st + 128 + 576 * c + r * 32 + ((half ^ ((r >> 2) & 1)) * 16));
+      const uint4 t = *reinterpret_cast<const uint4*>(st + 128 + 576 * c + 16 * lane);  // MMA fragment order
+      a[c][0] = t.x;
+      a[c][1] = t.y;
+      a[c][2] = t.z;
+      a[c][3] = t.w;
       meta[c] = reinterpret_cast<const uint32_t*>(st + 640 + 576 * c)[g * 2 + (lane & 1)];
     }
-    const uint8_t* B = st + REC;
+    // The tensor cores truncate as they add to an accumulator, so a tile starts from zero (low
+    // parts of the panel before the high ones) and joins the item's sum in a rounding add:
+    // over the thousands of samples of a central grid cell that halves the operator's noise.
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) {
-      uint32_t b[4];
-      ldmatrix_x4_trans(b, B + lane * BYTES + chunk_swizzle<CH>(nb, lane) * 16);
-      const int ai = SPLIT ? (nb % NA) : nb;
+    for (int na = 0; na < NA; ++na) {
+      float t[NCOMP][4];
 #pragma unroll
-      for (int c = 0; c < NCOMP; ++c) mma_sp_16832(acc[c][ai], a[c], b, meta[c]);
+      for (int part = SPLIT ? 1 : 0; part >= 0; --part) {
+        uint32_t b[4];
+        ldmatrix_x4_trans_u32(b, ldm(na + part * NA) + stage * STAGE);
+#pragma unroll
+        for (int c = 0; c < NCOMP; ++c) {
+          if (part == (SPLIT ? 1 : 0)) mma_sp_16832_zero(t[c], a[c], b, meta[c]);
+          else mma_sp_16832(t[c], a[c], b, meta[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[c][na][j] += t[c][j];
     }
     int32_t rows[2] = {-1, -1};
     if (info.flags & kRecLast) {
       rows[0] = record_row(trow, info.flags, g);
       rows[1] = record_row(trow, info.flags, g + 8);
     }
-    __syncwarp();  // this stage is refilled by the next iteration's record copy
+    __syncwarp();  // this slot and stage are refilled by the next iteration's copies
     if (info.flags & kRecLast) {  // last tile of its item
       interp_finish_item<ROWH, NCOMP, NA, EPI, CONJ, SUMC>(acc, v, o, info, lane, rows, wrow, scale);
 #pragma unroll
@@ -329,41 +388,38 @@ __global__ void __launch_bounds__(kInterpWarps * 32) interp_mmasp_kernel(InterpV
     }
   };
   // Iterations k = -kRecAhead .. n-1, two commit groups each (empty when out of range):
-  // rec(k + R) then gat(k + Ga), with R = kRecAhead, Ga = kGatherAhead.  Tile k lives in
-  // stage (k + R) % kStages; unrolling by kStages makes every stage address a constant.
+  // rec(k + R) then gat(k + Ga), with R = kRecAhead, Ga = kGatherAhead.  Tile k lives in record
+  // slot (k + R) % NR and gather stage (k + R) % NG; unrolling by a multiple of both makes
+  // every address a constant.
   // After committing rec(k + R), the groups newer than rec(k + Ga) are gat(k + 2Ga - R)
   // and the 2(R - Ga) - 1 groups of the later iterations, so wait<2(R - Ga)> lands the
   // record the next gather reads; after committing gat(k + Ga), wait<2 Ga> lands gat(k).
-  for (int k0 = -kRecAhead; k0 < n; k0 += kStages) {
+  constexpr int UN = NR;
+  static_assert(NR % NG == 0, "slots of both rings are constants");
+  for (int k0 = -kRecAhead; k0 < n; k0 += UN) {
 #pragma unroll
-    for (int u = 0; u < kStages; ++u) {
+    for (int u = 0; u < UN; ++u) {
       const int k = k0 + u;
       if (k >= n) break;
-      issue_record(k + kRecAhead, ring + ((u + kRecAhead) % kStages) * STAGE);
+      issue_record(k + kRecAhead, (u + kRecAhead) % NR);
       cp_async_wait<2 * (kRecAhead - kGatherAhead)>();
       __syncwarp();
-      issue_gather(k + kGatherAhead, ring + ((u + kGatherAhead) % kStages) * STAGE);
+      issue_gather(k + kGatherAhead, (u + kGatherAhead) % NR, (u + kGatherAhead) % NG);
       cp_async_wait<2 * kGatherAhead>();
       __syncwarp();
-      if (k >= 0) compute(ring + u * STAGE);
+      if (k >= 0) compute(u % NR, u % NG);
     }
   }
   cp_async_wait<0>();
 }
 
-template <int ROWH, bool SPLIT, int NCOMP, int EPI, bool CONJ, int STAGES, bool SUMC = false>
-static void launch_interp_s(const InterpView& v, const __half* panel, const InterpOut& o, cudaStream_t s) {
-  const int blocks = (v.n_warps + kInterpWarps - 1) / kInterpWarps;
-  const size_t smem = static_cast<size_t>(kInterpWarps) * STAGES * (record_bytes(NCOMP) + 32 * ROWH * 2);
-  auto k = interp_mmasp_kernel<ROWH, SPLIT, NCOMP, EPI, CONJ, STAGES, SUMC>;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (blocks > 0) launch_k(k, blocks, kInterpWarps * 32, smem, s, v.programmatic != 0, v, panel, o);
-}
-
 template <int ROWH, bool SPLIT, int NCOMP, int EPI, bool CONJ, bool SUMC = false>
 static void launch_interp_t(const InterpView& v, const __half* panel, const InterpOut& o, cudaStream_t s) {
-  if (v.stages == 4) launch_interp_s<ROWH, SPLIT, NCOMP, EPI, CONJ, 4, SUMC>(v, panel, o, s);
-  else launch_interp_s<ROWH, SPLIT, NCOMP, EPI, CONJ, 3, SUMC>(v, panel, o, s);
+  const int blocks = (v.n_warps + kInterpWarps - 1) / kInterpWarps;
+  constexpr size_t smem = interp_smem(ROWH, NCOMP);
+  auto k = interp_mmasp_kernel<ROWH, SPLIT, NCOMP, EPI, CONJ, SUMC>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (blocks > 0) launch_k(k, blocks, kInterpWarps * 32, smem, s, v.programmatic != 0, v, panel, o);
 }
 
 template <int ROWH>
@@ -388,31 +444,26 @@ static void dispatch_epi(const InterpView& v, const __half* panel, int epi, bool
 
 static int sm_count();
 
-template <int ROWH, int NCOMP, int STAGES>
-static int resident_warps_s() {
-  const size_t smem = static_cast<size_t>(kInterpWarps) * STAGES * (record_bytes(NCOMP) + 32 * ROWH * 2);
-  auto k = interp_mmasp_kernel<ROWH, true, NCOMP, EPI_GRID, NCOMP == 2, STAGES>;
+template <int ROWH, int NCOMP>
+static int resident_warps_t() {
+  constexpr size_t smem = interp_smem(ROWH, NCOMP);
+  auto k = interp_mmasp_kernel<ROWH, true, NCOMP, EPI_GRID, NCOMP == 2>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kInterpWarps * 32, smem);
   return std::max(1, per_sm) * kInterpWarps * sm_count();
 }
 
-template <int ROWH, int NCOMP>
-static int resident_warps_t(int stages) {
-  return stages == 4 ? resident_warps_s<ROWH, NCOMP, 4>() : resident_warps_s<ROWH, NCOMP, 3>();
-}
-
-int interp_resident_warps(int rowh, int ncomp, int stages) {
+int interp_resident_warps(int rowh, int ncomp) {
   switch (rowh * 4 + ncomp) {
-    case 16 * 4 + 1: return resident_warps_t<16, 1>(stages);
-    case 16 * 4 + 2: return resident_warps_t<16, 2>(stages);
-    case 32 * 4 + 1: return resident_warps_t<32, 1>(stages);
-    case 32 * 4 + 2: return resident_warps_t<32, 2>(stages);
-    case 48 * 4 + 1: return resident_warps_t<48, 1>(stages);
-    case 48 * 4 + 2: return resident_warps_t<48, 2>(stages);
-    case 64 * 4 + 1: return resident_warps_t<64, 1>(stages);
-    default: return resident_warps_t<64, 2>(stages);
+    case 16 * 4 + 1: return resident_warps_t<16, 1>();
+    case 16 * 4 + 2: return resident_warps_t<16, 2>();
+    case 32 * 4 + 1: return resident_warps_t<32, 1>();
+    case 32 * 4 + 2: return resident_warps_t<32, 2>();
+    case 48 * 4 + 1: return resident_warps_t<48, 1>();
+    case 48 * 4 + 2: return resident_warps_t<48, 2>();
+    case 64 * 4 + 1: return resident_warps_t<64, 1>();
+    default: return resident_warps_t<64, 2>();
   }
 }
 
@@ -1035,9 +1086,11 @@ static size_t fft_rows_bytes() {
 // two CTAs still fit on an SM with them; larger lines read them from global memory.
 constexpr size_t kFftStageSmem = 114 * 1024;
 
+// Dynamic shared memory beyond the default 48 KB, of which the kernels' static arrays take up
+// to 2 KB, has to be asked for.
 template <class K>
 static void ensure_smem(K k, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (bytes > 46 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
 static int sm_count() {

@@ -28,9 +28,13 @@ struct CgState {
 
 // Interpolation view on the device: AoS tile records, in the order the persistent warps
 // stream them (warp w owns records [warp_ranges[w].x, warp_ranges[w].y))
-//   [0,128)                  int32 gather row per column (internal panel row), -1 = dead
-//                            column (all coefficients zero: zero-filled, never read)
-//   [128+576c, +512)         f16 compressed A of component c, [16][16]
+//   [0,128)                  u32 byte offset of each gathered panel row, in lane order: entry j
+//                            of lane group q (gather_lanes lanes) is at q * gather_lanes + j
+//                            and stands for tile column gather_column(rowh, q, j);
+//                            kGatherDead = dead column (all coefficients zero: zero-filled,
+//                            never read)
+//   [128+576c, +512)         f16 compressed A of component c as mma.sp fragments: lane l holds
+//                            A[l / 4 + 8 (i & 1)][8 (i >> 1) + 2 (l % 4) ..+1], i < 4, at 16 l
 //   [640+576c, +64)          u32 mma.sp pair metadata of component c, [16]
 //   [128+576n, +16)          RecordInfo (n = component count)
 //   [128+576n+16, +48)       24-bit output row of each of the 16 tile rows (little endian;
@@ -57,6 +61,13 @@ struct RecordInfo {
   int32_t chunk;       // chunk index | nchunks << 16
 };
 static_assert(sizeof(RecordInfo) == 16, "record info is 16 bytes");
+constexpr uint32_t kGatherDead = 16;  // offsets are multiples of 32: the bit is free, and the
+                                      // address it makes is inside the panel, though never read
+// Lanes that share a gathered row of 2 rowh bytes, and so the rows each lane gathers: a whole
+// row of 16-byte chunks when that is a power of two, else a 32-byte sector of it.
+__host__ __device__ constexpr int gather_lanes(int rowh) { return rowh == 48 ? 2 : rowh / 8; }
+// tile column whose row lane group q (of 32 / gather_lanes) gathers j-th
+__host__ __device__ constexpr int gather_column(int rowh, int q, int j) { return q + j * (32 / gather_lanes(rowh)); }
 __host__ __device__ constexpr int record_bytes(int ncomp) { return 128 + 576 * ncomp + kRecInfoBytes; }
 
 struct InterpView {
@@ -68,7 +79,6 @@ struct InterpView {
   int32_t groups = 0;
   int32_t ncomp = 0;
   int32_t rec_bytes = 0;
-  int32_t stages = 3;                   // per-warp ring depth: 3, or 4 when the gathered panel exceeds L2
   int32_t programmatic = 1;             // 1: launched with programmatic dependent launch (0 for the
                                         //    1/share slices of batched cases, which share the SMs)
   int32_t sum_components = 0;           // 1: the two components are a real coefficient's FP16 high and
@@ -156,7 +166,7 @@ void launch_interp_tc(const InterpTcView& v, const __half* panel, int epi, const
 size_t interp_tc_smem_bytes();
 // warps the persistent interpolation kernel keeps resident on this device for a panel row
 // width / component count (used to cut the item list into per-warp runs)
-int interp_resident_warps(int rowh, int ncomp, int stages);
+int interp_resident_warps(int rowh, int ncomp);
 constexpr int kInterpWarpsPerCta = 4;
 
 void launch_norm_partials(const float2* v, int64_t n, double* part, cudaStream_t s);

@@ -394,14 +394,13 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
   // poles, first in their run) is followed by whole small groups up to the average run length,
   // so runs can be cut close to the average instead of at multiples of the chunk length.
   const bool large_panel = h.n_cols * 8 * static_cast<int64_t>(P->C) > kLocalityPanelBytes;
-  const int stages = large_panel ? 4 : 3;
   if (large_panel) {
     items.insert(items.end(), small.begin(), small.end());
   } else {
     int64_t total = 0;
     for (const Item& it : items) total += it.t1 - it.t0;
     for (const Item& it : small) total += it.t1 - it.t0;
-    const int warps_full = interp_resident_warps(4 * P->C, ncomp, stages);
+    const int warps_full = interp_resident_warps(4 * P->C, ncomp);
     const double avg = static_cast<double>(total) / std::max(1, warps_full);
     std::vector<Item> order;
     order.reserve(items.size() + small.size());
@@ -419,6 +418,7 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
   }
   // persistent warps: contiguous runs of items with about the same number of tiles each;
   // records are stored in that stream order so each warp reads one contiguous range
+  const int rowh = 4 * P->C, lanes = gather_lanes(rowh);
   std::vector<uint8_t> records(static_cast<size_t>(tiles) * rec, 0);
   d.item_ends.clear();
   int64_t pos = 0;
@@ -426,20 +426,20 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
     for (uint32_t t = it.t0; t < it.t1; ++t, ++pos) {
       uint8_t* r = records.data() + pos * rec;
       const uint32_t live = live_columns(h, t);
-      int32_t cols[kKTile];
-      for (int j = 0; j < kKTile; ++j) {
-        int64_t c = h.tile_col_ids[t * kKTile + j];
-        if (cols_are_cells) c = to_internal(P, c);
-        cols[j] = ((live >> j) & 1u) ? static_cast<int32_t>(c) : -1;
-      }
-      std::memcpy(r, cols, sizeof cols);
+      uint32_t offsets[kKTile];
+      for (int q = 0; q < kKTile / lanes; ++q)
+        for (int j = 0; j < lanes; ++j) {
+          const int col = gather_column(rowh, q, j);
+          int64_t c = h.tile_col_ids[static_cast<size_t>(t) * kKTile + col];
+          if (cols_are_cells) c = to_internal(P, c);
+          offsets[q * lanes + j] = ((live >> col) & 1u) ? static_cast<uint32_t>(c * rowh * 2) : kGatherDead;
+        }
+      std::memcpy(r, offsets, sizeof offsets);
       for (int c = 0; c < ncomp; ++c) {
-        // A: 16 rows of 32 B; the two 16-B halves of row r are swapped when (r >> 2) & 1 so
-        // ldmatrix reads 8 rows of one half without shared-memory bank conflicts
-        for (int row = 0; row < 16; ++row)
-          for (int half = 0; half < 2; ++half)
-            std::memcpy(r + 128 + 576 * c + row * 32 + ((half ^ ((row >> 2) & 1)) * 16),
-                        &h.a[c][t * 256 + row * 16 + half * 8], 16);
+        const uint16_t* a = &h.a[c][static_cast<size_t>(t) * 256];
+        for (int l = 0; l < 32; ++l)
+          for (int i = 0; i < 4; ++i)
+            std::memcpy(r + 128 + 576 * c + 16 * l + 4 * i, a + (l / 4 + 8 * (i & 1)) * 16 + 8 * (i >> 1) + 2 * (l % 4), 4);
         std::memcpy(r + 640 + 576 * c, &h.meta[c][t * 16], 64);
       }
       RecordInfo info;
@@ -461,7 +461,7 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
     d.item_ends.push_back(pos);
   }
   if (pos != tiles) fail(TSN_ERR_FORMAT, "group offsets do not cover the tiles");
-  const std::vector<int2> ranges = cut_ranges(d.item_ends, tiles, interp_resident_warps(4 * P->C, ncomp, stages));
+  const std::vector<int2> ranges = cut_ranges(d.item_ends, tiles, interp_resident_warps(4 * P->C, ncomp));
   if (P->use_tc && !target) build_tc_steps(P, d, h, rows_are_cells, cols_are_cells);
   d.records.upload(records);
   d.counters.upload(std::vector<int32_t>(std::max(nsplit, 1), 0));
@@ -475,7 +475,6 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
   d.v.groups = static_cast<int32_t>(groups);
   d.v.ncomp = ncomp;
   d.v.rec_bytes = rec;
-  d.v.stages = stages;
   d.tiles = tiles;
   d.groups = groups;
   d.active_rows = h.active_rows;
@@ -1084,7 +1083,7 @@ void prepare_share(tsn_plan* P, int share) {
   if (share <= 1) return;
   for (DevView& d : P->view) {
     if (!d.present || d.share == share) continue;
-    const int warps = std::max(kInterpWarpsPerCta, interp_resident_warps(4 * P->C, d.v.ncomp, d.v.stages) / share);
+    const int warps = std::max(kInterpWarpsPerCta, interp_resident_warps(4 * P->C, d.v.ncomp) / share);
     const std::vector<int2> ranges = cut_ranges(d.item_ends, d.tiles, warps);
     d.ranges_shared.upload(ranges);
     d.v_shared = d.v;
@@ -1725,27 +1724,35 @@ tsn_status tsn_interp_component(tsn_plan* plan, int32_t view, int32_t component,
     // cell_to_internal is an involution on square grids: internal row j holds reference row map[j]
     launch_gather_rows_f16(static_cast<const __half*>(dense_f16), cm.as<int32_t>(), d.n_cols, 16, din.as<__half>(), s);
     InterpView v = d.v;
-    std::vector<uint8_t> dummy;
     InterpOut o;
     o.raw = dout.as<float>();
     o.rows = d.output_size;
-    // component selection: a two-component view gets a single-component record copy
-    // (columns | A and metadata of the component | record info and rows)
-    DeviceBuffer shifted;
-    if (d.v.ncomp == 2) {
-      const int one_rec = record_bytes(1);
+    // single-component records (columns | A and metadata of the component | record info and
+    // rows) whose offsets are those of 16-channel rows
+    DeviceBuffer narrow;
+    {
+      const int one_rec = record_bytes(1), rowh = 4 * plan->C, lanes = gather_lanes(rowh), lanes16 = gather_lanes(16);
       std::vector<uint8_t> host(static_cast<size_t>(d.tiles) * d.v.rec_bytes);
       CUDA_OK(cudaMemcpy(host.data(), d.v.records, host.size(), cudaMemcpyDeviceToHost));
       std::vector<uint8_t> one(static_cast<size_t>(d.tiles) * one_rec);
       for (int64_t t = 0; t < d.tiles; ++t) {
         const uint8_t* src = &host[t * d.v.rec_bytes];
         uint8_t* dst = &one[t * one_rec];
-        std::memcpy(dst, src, 128);
+        uint32_t in[kKTile], cols[kKTile], out16[kKTile];
+        std::memcpy(in, src, sizeof in);
+        for (int q = 0; q < kKTile / lanes; ++q)
+          for (int j = 0; j < lanes; ++j) {
+            const uint32_t o = in[q * lanes + j];
+            cols[gather_column(rowh, q, j)] = o == kGatherDead ? o : o / static_cast<uint32_t>(rowh * 2) * 32;
+          }
+        for (int q = 0; q < kKTile / lanes16; ++q)
+          for (int j = 0; j < lanes16; ++j) out16[q * lanes16 + j] = cols[gather_column(16, q, j)];
+        std::memcpy(dst, out16, sizeof out16);
         std::memcpy(dst + 128, src + 128 + 576 * component, 576);
-        std::memcpy(dst + 128 + 576, src + 128 + 576 * 2, kRecInfoBytes);
+        std::memcpy(dst + 128 + 576, src + 128 + 576 * d.v.ncomp, kRecInfoBytes);
       }
-      shifted.upload(one);
-      v.records = shifted.as<uint8_t>();
+      narrow.upload(one);
+      v.records = narrow.as<uint8_t>();
       v.rec_bytes = one_rec;
     }
     v.ncomp = 1;
