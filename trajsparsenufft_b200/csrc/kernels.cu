@@ -24,20 +24,23 @@ namespace tsn {
 
 using namespace dev;
 
-// The warp interpolation is launched with programmatic stream serialization: its CTAs start
-// (launch, shared-memory carve-up, the first plan-record copies) while the kernel ahead of it
-// in the stream drains, and wait in pdl_wait before touching its results. Every kernel of the
-// CG iteration calls pdl_trigger once it has passed its own wait, so the interpolation behind
-// it may launch then. On the 256^2 / 8-coil headline solve this took a CG iteration from 71.8
-// to 69.5 us. Batched cases, whose kernels run side by side on slices of the GPU, launch it
-// plainly: early CTAs would wait beside the other cases' kernels (the 48-case batch measured
-// 1191 recons/s with it, 1325-1390 without it on other boxes; 1329 plain vs 1325 with every
-// launch plain on one box). The FFT stages are launched plainly: their CTAs, started early beside a kernel
-// that leaves room on the SMs (the row stages hold ~1.7 of 3 CTAs per SM; the interpolation
-// leaves room for one more), made the solve 3-9% slower although each stage timed alone
-// back to back got faster. They keep the same prologue split (plan rows before pdl_wait) for
-// when they are. TSN_PDL=0 in the environment launches everything plainly (same results,
-// bit for bit).
+// Programmatic dependent launch (the next kernel's CTAs start while this one drains, and wait
+// in pdl_wait before they touch its results; every kernel launched so calls pdl_wait).
+//
+// Inside the solver's graph only the interpolation is launched so: a plain graph edge costs
+// 0.65 us, and FFT stages that start early wait beside a kernel that leaves room on the SMs
+// (10-iteration solves, plain / programmatic FFT stages: 256^2 x 8 coils 616 / 636 us, 128^2 x
+// 4 coils 302 / 309 us). The kernel ahead of an interpolation calls pdl_trigger after its own
+// wait; the others leave it to their end. Batched cases, whose kernels run side by side on
+// slices of the GPU, launch everything plainly: early CTAs would wait beside the other cases'
+// kernels (the 48-case batch measured 1191 recons/s with it, 1325-1390 without it).
+//
+// Direct calls launch every kernel so: a plain launch behind a running kernel costs about 2 us
+// and rounds the period up to the next 2 us (kernels of 2.5 us follow each other at 5.1 us),
+// a programmatic one 0.7 us.
+//
+// TSN_PDL=0 in the environment launches everything plainly (the results are the same bit for
+// bit).
 static bool pdl_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("TSN_PDL");
@@ -487,6 +490,7 @@ void launch_interp(const InterpView& v, const __half* panel, int rowh, bool spli
 // ------------------------------------------------------------------------------------------
 __global__ void norm_partials_kernel(const float2* __restrict__ v, int64_t n, double* __restrict__ part) {
   __shared__ double scratch[33];
+  pdl_wait();
   double acc = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -497,8 +501,8 @@ __global__ void norm_partials_kernel(const float2* __restrict__ v, int64_t n, do
   if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
-void launch_norm_partials(const float2* v, int64_t n, double* part, cudaStream_t s) {
-  norm_partials_kernel<<<kNormParts, 256, 0, s>>>(v, n, part);
+void launch_norm_partials(const float2* v, int64_t n, double* part, cudaStream_t s, bool pdl) {
+  launch_k(norm_partials_kernel, kNormParts, 256, 0, s, pdl, v, n, part);
 }
 
 // Sum of nparts partials, identical (fixed tree) in every block. Call with all threads.
@@ -604,9 +608,9 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
     }
     cp_async_commit();
   };
-  if (blockIdx.x < lines) issue(blockIdx.x, 1);
+  if (f.maps_early && blockIdx.x < lines) issue(blockIdx.x, 1);
   pdl_wait();
-  pdl_trigger();
+  if (!f.maps_early && blockIdx.x < lines) issue(blockIdx.x, 1);
   if (blockIdx.x < lines) issue(blockIdx.x, 2);
   double total, alpha = 0.0, rho_prev = 0.0;
   if (mode == 4) {  // finish iteration iter-1 (the cg_update scalars)
@@ -746,7 +750,6 @@ fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1, float2* __restrict__ z2
   float2* buf = reinterpret_cast<float2*>(sm);
   const int N = f.N, items = N * G * GROUPS;
   pdl_wait();
-  pdl_trigger();
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
     const int q2 = t / N, i0 = t - q2 * N;
@@ -773,6 +776,7 @@ __global__ void split_samples_kernel(const float2* __restrict__ y, const float* 
                                      int C, __half* __restrict__ panel, const double* __restrict__ parts, int nparts,
                                      CgState* __restrict__ st) {
   __shared__ double red[33];
+  pdl_wait();
   const double total = sum_partials(parts, nparts, red);
   const float sigma = pow2_scale(total, static_cast<double>(m) * C, kPanelTarget);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -811,7 +815,6 @@ inv_cols_kernel(FftArgs f, const float2* __restrict__ grid, float2* __restrict__
   float2* buf = reinterpret_cast<float2*>(sm);
   const int N = f.N, items = f.gcols() * GROUPS;
   pdl_wait();
-  pdl_trigger();
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
     if (it != blockIdx.x) __syncthreads();
@@ -843,7 +846,6 @@ inv_mid_kernel(FftArgs f, const float2* __restrict__ z2, float2* __restrict__ z1
   float2* buf = reinterpret_cast<float2*>(sm);
   const int N = f.N, items = G * N * GROUPS;
   pdl_wait();
-  pdl_trigger();
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
     const int q2 = t / N, i0 = t - q2 * N;
@@ -909,7 +911,6 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
   };
   if (blockIdx.x < lines) issue(blockIdx.x, 1);
   pdl_wait();
-  pdl_trigger();
   if (blockIdx.x < lines) issue(blockIdx.x, 2);
   float factor;
   if (mode == 2) factor = f.gs() / st->sigma[iter] * inv_scale2;
@@ -1147,7 +1148,7 @@ void launch_fwd_rows(const FftArgs& f, const float2* x, float2* z1, int mode, fl
     constexpr int T = LineFft<GG, CC, false>::THREADS;
     auto k = fwd_rows_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, false, f, x, z1, mode, p, r, partials, nparts, st,
+    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, f.pdl, f, x, z1, mode, p, r, partials, nparts, st,
              iter, xs, ap, stage);
   }));
 }
@@ -1158,7 +1159,7 @@ void launch_fwd_cols(const FftArgs& f, const float2* z1, __half* panel, cudaStre
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = fwd_cols_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, false, f, z1, panel);
+    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, f.pdl, f, z1, panel);
   }));
 }
 
@@ -1168,7 +1169,7 @@ void launch_fwd_mid(const FftArgs& f, const float2* z1, float2* z2, cudaStream_t
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = fwd_mid_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, false, f, z1, z2);
+    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, f.pdl, f, z1, z2);
   }));
 }
 
@@ -1178,15 +1179,15 @@ void launch_inv_mid(const FftArgs& f, const float2* z2, float2* z1, cudaStream_t
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = inv_mid_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, false, f, z2, z1);
+    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, f.pdl, f, z2, z1);
   }));
 }
 
 void launch_split_samples(const float2* y, const float* density, int64_t m, int c, __half* panel,
-                          const double* partials, int nparts, CgState* st, cudaStream_t s) {
+                          const double* partials, int nparts, CgState* st, cudaStream_t s, bool pdl) {
   const int64_t blocks = std::min<int64_t>((m * (c / 4) + 255) / 256, 8 * 148);
-  split_samples_kernel<<<static_cast<int>(std::max<int64_t>(blocks, 1)), 256, 0, s>>>(y, density, m, c, panel, partials,
-                                                                                        nparts, st);
+  launch_k(split_samples_kernel, static_cast<int>(std::max<int64_t>(blocks, 1)), 256, 0, s, pdl, y, density, m, c, panel,
+           partials, nparts, st);
 }
 
 void launch_inv_cols(const FftArgs& f, const float2* grid, float2* w1, cudaStream_t s) {
@@ -1195,7 +1196,7 @@ void launch_inv_cols(const FftArgs& f, const float2* grid, float2* w1, cudaStrea
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = inv_cols_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, false, f, grid, w1);
+    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, f.pdl, f, grid, w1);
   }));
 }
 
@@ -1211,7 +1212,7 @@ void launch_inv_rows(const FftArgs& f, const float2* w1, float2* out, int mode, 
     constexpr int T = LineFft<GG, CC, true>::THREADS;
     auto k = inv_rows_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, false, f, w1, out, mode, x, r, p, partials, st, iter,
+    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, f.pdl, f, w1, out, mode, x, r, p, partials, st, iter,
              inv_scale2, lambda_scaled, static_cast<int>(region), epi_smem);
   }));
 }
@@ -1228,19 +1229,21 @@ void launch_cg_finish(int nparts, const double* rr_parts, CgState* st, int iters
 // Block b sums section b (part + b * stride, n values) into its first value.
 __global__ void reduce_partials_kernel(double* part, int n, int64_t stride) {
   __shared__ double red[33];
+  pdl_wait();
   double* sec = part + blockIdx.x * stride;
   const double t = sum_partials(sec, n, red);  // every read lands before block_sum's first barrier
   if (threadIdx.x == 0) sec[0] = t;
 }
 
-void launch_reduce_partials(double* part, int n, cudaStream_t s, int sections, int64_t stride) {
-  reduce_partials_kernel<<<sections, 1024, 0, s>>>(part, n, stride);
+void launch_reduce_partials(double* part, int n, cudaStream_t s, int sections, int64_t stride, bool pdl) {
+  launch_k(reduce_partials_kernel, sections, 1024, 0, s, pdl, part, n, stride);
 }
 
 // FP64 partials of Re <a, b> over n complex values (grid-stride, one per block).
 __global__ void rdot_partials_kernel(const float2* __restrict__ a, const float2* __restrict__ b, int64_t n,
                                      double* __restrict__ part) {
   __shared__ double scratch[33];
+  pdl_wait();
   double acc = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -1254,17 +1257,18 @@ __global__ void rdot_partials_kernel(const float2* __restrict__ a, const float2*
 // out[0] = the sum of n partials, in a fixed order (one block).
 __global__ void sum_partials_to_kernel(const double* __restrict__ part, int n, double* __restrict__ out) {
   __shared__ double red[33];
+  pdl_wait();
   const double t = sum_partials(part, n, red);
   if (threadIdx.x == 0) out[0] = t;
 }
 
-void launch_rdot(const float2* a, const float2* b, int64_t n, double* parts, double* out, cudaStream_t s) {
-  rdot_partials_kernel<<<kNormParts, 256, 0, s>>>(a, b, n, parts);
-  sum_partials_to_kernel<<<1, 256, 0, s>>>(parts, kNormParts, out);
+void launch_rdot(const float2* a, const float2* b, int64_t n, double* parts, double* out, cudaStream_t s, bool pdl) {
+  launch_k(rdot_partials_kernel, kNormParts, 256, 0, s, pdl, a, b, n, parts);
+  launch_k(sum_partials_to_kernel, 1, 256, 0, s, pdl, parts, kNormParts, out);
 }
 
-void launch_sum_partials_to(const double* parts, int n, double* out, cudaStream_t s) {
-  sum_partials_to_kernel<<<1, 256, 0, s>>>(parts, n, out);
+void launch_sum_partials_to(const double* parts, int n, double* out, cudaStream_t s, bool pdl) {
+  launch_k(sum_partials_to_kernel, 1, 256, 0, s, pdl, parts, n, out);
 }
 
 // ---- reverse-mode CG step (the adjoint recurrences of one CG iteration) -------------------
@@ -1285,6 +1289,7 @@ __global__ void cgb_dots_kernel(int64_t n, const float2* __restrict__ rb, const 
                                 const float2* __restrict__ rn, const float2* __restrict__ xb,
                                 double* __restrict__ parts) {
   __shared__ double red[165];
+  pdl_wait();
   double d[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -1326,6 +1331,7 @@ __global__ void cgb_update_kernel(int64_t n, int nparts, const double* __restric
                                   float2* __restrict__ qb, double* __restrict__ qnorm_parts) {
   __shared__ double red[132];
   __shared__ double dl[5];
+  pdl_wait();
   const double4 s4 = sum_partials4(parts, nparts, nparts, red);
   if (threadIdx.x == 0) {
     dl[0] = s4.x;
@@ -1366,6 +1372,7 @@ __global__ void cgb_finish_kernel(int64_t n, int coils, float2* __restrict__ pb,
                                   const float2* __restrict__ qb, const float2* __restrict__ t,
                                   const float2* __restrict__ tb, const float2* __restrict__ p,
                                   float2* __restrict__ sb) {
+  pdl_wait();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float2 vm = mqb[i];
@@ -1395,6 +1402,7 @@ __global__ void cgf_update_kernel(int64_t n, const double* __restrict__ rho_p, c
                                   const float2* __restrict__ r, const float2* __restrict__ q,
                                   float2* __restrict__ x_out, float2* __restrict__ r_out, double* __restrict__ parts) {
   __shared__ double red[33];
+  pdl_wait();
   const double a = *rho_p / *gamma_p;
   double acc = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -1419,6 +1427,7 @@ __global__ void cgf_direction_kernel(int64_t n, int nparts, const double* __rest
                                      const float2* __restrict__ p, const float2* __restrict__ r_new,
                                      float2* __restrict__ p_out, double* __restrict__ pnorm_parts) {
   __shared__ double red[33];
+  pdl_wait();
   const double rho_n = sum_partials(parts, nparts, red);
   if (blockIdx.x == 0 && threadIdx.x == 0) *rho_out = rho_n;
   const double b = rho_n / *rho_p;
@@ -1438,23 +1447,24 @@ __global__ void cgf_direction_kernel(int64_t n, int nparts, const double* __rest
 
 void launch_cg_step(int64_t n, double* parts, const double* rho, const double* gamma, const float2* x, const float2* p,
                     const float2* r, const float2* q, float2* x_out, float2* r_out, float2* p_out, double* rho_out,
-                    double* p_norm_parts, cudaStream_t s) {
-  cgf_update_kernel<<<kCgbBlocks, 256, 0, s>>>(n, rho, gamma, x, p, r, q, x_out, r_out, parts);
-  cgf_direction_kernel<<<kCgbBlocks, 256, 0, s>>>(n, kCgbBlocks, parts, rho, rho_out, p, r_out, p_out, p_norm_parts);
+                    double* p_norm_parts, cudaStream_t s, bool pdl) {
+  launch_k(cgf_update_kernel, kCgbBlocks, 256, 0, s, pdl, n, rho, gamma, x, p, r, q, x_out, r_out, parts);
+  launch_k(cgf_direction_kernel, kCgbBlocks, 256, 0, s, pdl, n, kCgbBlocks, parts, rho, rho_out, p, r_out, p_out,
+           p_norm_parts);
 }
 
 void launch_cg_adjoint_step(int64_t n, double* parts, const double* rho, const double* rho_n, const double* gamma,
                             const double* rhob, double* rhob_out, float2* rb, float2* pb, const float2* p,
                             const float2* q, const float2* rn, const float2* xb, float2* qb, double* qb_norm_parts,
-                            cudaStream_t s) {
-  cgb_dots_kernel<<<kCgbBlocks, 256, 0, s>>>(n, rb, pb, p, q, rn, xb, parts);
-  cgb_update_kernel<<<kCgbBlocks, 256, 0, s>>>(n, kCgbBlocks, parts, rho, rho_n, gamma, rhob, rhob_out, rb, pb, p, q,
-                                                rn, xb, qb, qb_norm_parts);
+                            cudaStream_t s, bool pdl) {
+  launch_k(cgb_dots_kernel, kCgbBlocks, 256, 0, s, pdl, n, rb, pb, p, q, rn, xb, parts);
+  launch_k(cgb_update_kernel, kCgbBlocks, 256, 0, s, pdl, n, kCgbBlocks, parts, rho, rho_n, gamma, rhob, rhob_out, rb, pb,
+           p, q, rn, xb, qb, qb_norm_parts);
 }
 
 void launch_cg_adjoint_finish(int64_t n, int coils, float2* pb, const float2* mqb, const float2* qb, const float2* t,
-                              const float2* tb, const float2* p, float2* sb, cudaStream_t s) {
-  cgb_finish_kernel<<<kCgbBlocks, 256, 0, s>>>(n, coils, pb, mqb, qb, t, tb, p, sb);
+                              const float2* tb, const float2* p, float2* sb, cudaStream_t s, bool pdl) {
+  launch_k(cgb_finish_kernel, kCgbBlocks, 256, 0, s, pdl, n, coils, pb, mqb, qb, t, tb, p, sb);
 }
 
 template <class T>

@@ -107,6 +107,9 @@ struct FftArgs {
   const float2* smaps = nullptr;        // [C][N]^dims or null
   int share = 1;                        // persistent grids use 1/share of the resident CTAs
   int dims = 2;                         // 2: image [N][N]; 3: volume [N][N][N]
+  bool pdl = false;                     // launch with programmatic dependent launch (direct calls)
+  bool maps_early = true;               // forward rows may read the coil maps ahead of pdl_wait: a kernel of
+                                        // this call has already waited for the caller's work
   // image lines along the last axis (items of the row stages)
   __host__ __device__ int lines() const { return dims == 3 ? N * N : N; }
   // pixels (voxels) of one image
@@ -169,7 +172,8 @@ size_t interp_tc_smem_bytes();
 int interp_resident_warps(int rowh, int ncomp);
 constexpr int kInterpWarpsPerCta = 4;
 
-void launch_norm_partials(const float2* v, int64_t n, double* part, cudaStream_t s);
+// pdl, here and below: launch with programmatic dependent launch (FftArgs::pdl)
+void launch_norm_partials(const float2* v, int64_t n, double* part, cudaStream_t s, bool pdl = false);
 
 // Stage layouts (images: i0 slow, i1 fast; volumes: i0, i1, i2; grids in internal rows
 // q1*G + q0 for images, (q2*G + q1)*G + q0 for volumes):
@@ -195,10 +199,10 @@ void launch_fwd_mid(const FftArgs& f, const float2* z1, float2* z2, cudaStream_t
 void launch_inv_mid(const FftArgs& f, const float2* z2, float2* z1, cudaStream_t s);
 // totals of `sections` runs of n partials (stride apart) into each run's first value, one CTA
 // per run in a fixed order
-void launch_reduce_partials(double* part, int n, cudaStream_t s, int sections = 1, int64_t stride = 0);
+void launch_reduce_partials(double* part, int n, cudaStream_t s, int sections = 1, int64_t stride = 0, bool pdl = false);
 // samples [C][M] (scaled by sigma_y, density) -> sample panel [M][4C]
 void launch_split_samples(const float2* y, const float* density, int64_t m, int c, __half* panel,
-                          const double* partials, int nparts, CgState* st, cudaStream_t s);
+                          const double* partials, int nparts, CgState* st, cudaStream_t s, bool pdl = false);
 // inverse columns: grid [G^dims][C] -> w1 [G][N][C] (images) or z2 (volumes)
 void launch_inv_cols(const FftArgs& f, const float2* grid, float2* w1, cudaStream_t s);
 // inverse rows + crop + deapod + coil combine
@@ -221,25 +225,26 @@ void launch_cg_update(int N, int lines, int nparts, float2* x, float2* r, const 
                       const double* pap_parts, double* rr_parts, CgState* st, int iter, cudaStream_t s);
 void launch_cg_finish(int nparts, const double* rr_parts, CgState* st, int iters, cudaStream_t s);
 // out[0] = Re <a, b> over n complex values in FP64 (kNormParts partials in parts, fixed order)
-void launch_rdot(const float2* a, const float2* b, int64_t n, double* parts, double* out, cudaStream_t s);
+void launch_rdot(const float2* a, const float2* b, int64_t n, double* parts, double* out, cudaStream_t s,
+                 bool pdl = false);
 // out[0] = the sum of n partials in a fixed order
-void launch_sum_partials_to(const double* parts, int n, double* out, cudaStream_t s);
+void launch_sum_partials_to(const double* parts, int n, double* out, cudaStream_t s, bool pdl = false);
 // Forward CG step on caller-owned vectors: alpha = rho / gamma, x_out = x + alpha p (x may be
 // null), r_out = r - alpha q, rho_out = |r_out|^2 (FP64, 296 partials in parts, fixed order),
 // p_out = r_out + (rho_out / rho) p.
 void launch_cg_step(int64_t n, double* parts, const double* rho, const double* gamma, const float2* x, const float2* p,
                     const float2* r, const float2* q, float2* x_out, float2* r_out, float2* p_out, double* rho_out,
-                    double* p_norm_parts, cudaStream_t s);
+                    double* p_norm_parts, cudaStream_t s, bool pdl = false);
 constexpr int kCgStepParts = 296;  // FP64 partials of the CG-step kernels (one per block)
 // Reverse-mode CG step (kernels.cu): five FP64 inner products in one pass (parts: 5 x 296
 // doubles), then rb, pb updated in place, qb written and rhob of the step to *rhob_out.
 void launch_cg_adjoint_step(int64_t n, double* parts, const double* rho, const double* rho_n, const double* gamma,
                             const double* rhob, double* rhob_out, float2* rb, float2* pb, const float2* p,
                             const float2* q, const float2* rn, const float2* xb, float2* qb, double* qb_norm_parts,
-                            cudaStream_t s);
+                            cudaStream_t s, bool pdl = false);
 // pb += mqb and, with sb given, the coil-map cotangent sb[c] += conj(qb) t[c] + tb[c] conj(p).
 void launch_cg_adjoint_finish(int64_t n, int coils, float2* pb, const float2* mqb, const float2* qb, const float2* t,
-                              const float2* tb, const float2* p, float2* sb, cudaStream_t s);
+                              const float2* tb, const float2* p, float2* sb, cudaStream_t s, bool pdl = false);
 
 void launch_gather_rows_f16(const __half* src, const int32_t* map, int64_t rows, int width, __half* dst,
                             cudaStream_t s);

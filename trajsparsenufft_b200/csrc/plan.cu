@@ -576,8 +576,20 @@ void allocate_workspaces(tsn_plan* P) {
   CUDA_OK(cudaGetLastError());
 }
 
-FftArgs fft_args(const tsn_plan* P, const void* smaps, int share = 1) {
+// Whether a direct call launches its kernels with programmatic dependent launch: yes, unless
+// the caller's stream is being captured (plain graph edges are as short, see kernels.cu).
+bool direct_pdl(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();  // another thread captures the legacy stream: plain launches
+    return false;
+  }
+  return st == cudaStreamCaptureStatusNone;
+}
+
+FftArgs fft_args(const tsn_plan* P, const void* smaps, int share = 1, bool pdl = false) {
   FftArgs f;
+  f.pdl = pdl;
   f.share = share;
   f.N = P->N;
   f.G = P->G;
@@ -617,10 +629,10 @@ void inv_to_lines(tsn_plan* P, const FftArgs& f, const float2* grid, cudaStream_
 // Partials written per image line are summed once for volumes (N^2 of them would be re-read
 // by every CTA of the next stage); returns how many partials the consumer reads. `sections`
 // runs of partials, one line count apart, are summed in one launch.
-int settle_partials(const tsn_plan* P, double* parts, cudaStream_t s, int sections = 1) {
+int settle_partials(const tsn_plan* P, double* parts, cudaStream_t s, int sections = 1, bool pdl = false) {
   if (P->dims != 3) return P->N;
   const int64_t lines = image_pixels(P) / P->N;
-  launch_reduce_partials(parts, static_cast<int>(lines), s, sections, lines);
+  launch_reduce_partials(parts, static_cast<int>(lines), s, sections, lines, pdl);
   return 1;
 }
 
@@ -1026,10 +1038,10 @@ void run_interp(const tsn_plan* P, int which, int share, int epi, const InterpOu
 }
 
 void enqueue_forward(tsn_plan* P, const void* x, const void* smaps, void* y, cudaStream_t s, bool reference = false) {
-  const FftArgs f = fft_args(P, smaps);
+  const FftArgs f = fft_args(P, smaps, 1, direct_pdl(s));
   CgState* st = P->state.as<CgState>();
   const int64_t n = image_pixels(P) * (smaps ? 1 : P->C);
-  launch_norm_partials(static_cast<const float2*>(x), n, P->norm_parts.as<double>(), s);
+  launch_norm_partials(static_cast<const float2*>(x), n, P->norm_parts.as<double>(), s, f.pdl);
   fwd_chain(P, f, static_cast<const float2*>(x), 0, nullptr, nullptr, P->norm_parts.as<double>(), kNormParts, st, 0,
             P->panel.as<__half>(), s);
   InterpOut o;
@@ -1050,11 +1062,12 @@ static_assert(kCgStepParts == TSN_CG_STEP_PARTS, "CG-step partial count of the k
 
 void enqueue_normal(tsn_plan* P, const void* p, const void* smaps, const float* density, float lambda, void* q,
                     void* coils, double* pq, const double* p_parts, int n_p_parts, cudaStream_t s) {
-  const FftArgs f = fft_args(P, smaps);
+  FftArgs f = fft_args(P, smaps, 1, direct_pdl(s));
+  f.maps_early = p_parts == nullptr;  // else the forward rows are the call's first kernel
   CgState* st = P->state.as<CgState>();
   const float2* pv = static_cast<const float2*>(p);
   if (!p_parts) {  // the panel scale of p from |p|^2 partials, unless the caller has them
-    launch_norm_partials(pv, image_pixels(P), P->norm_parts.as<double>(), s);
+    launch_norm_partials(pv, image_pixels(P), P->norm_parts.as<double>(), s, f.pdl);
     p_parts = P->norm_parts.as<double>();
     n_p_parts = kNormParts;
   }
@@ -1074,7 +1087,7 @@ void enqueue_normal(tsn_plan* P, const void* p, const void* smaps, const float* 
   double* parts = P->parts_rr.as<double>();
   launch_inv_rows(f, P->z1.as<float2>(), static_cast<float2*>(q), 5, static_cast<float2*>(coils), nullptr, pv, parts, st,
                   0, 1.0f, lambda, s);
-  if (pq) launch_sum_partials_to(parts, settle_partials(P, parts, s), pq, s);
+  if (pq) launch_sum_partials_to(parts, settle_partials(P, parts, s, 1, f.pdl), pq, s, f.pdl);
 }
 
 // Cuts (once per share value, outside any stream capture) the interpolation warp runs for a
@@ -1095,11 +1108,11 @@ void prepare_share(tsn_plan* P, int share) {
 }
 
 void enqueue_adjoint_grid(tsn_plan* P, const void* y, const float* density, cudaStream_t s, int share = 1,
-                          bool reference = false) {
+                          bool reference = false, bool pdl = false) {
   CgState* st = P->state.as<CgState>();
-  launch_norm_partials(static_cast<const float2*>(y), P->M * P->C, P->norm_parts.as<double>(), s);
+  launch_norm_partials(static_cast<const float2*>(y), P->M * P->C, P->norm_parts.as<double>(), s, pdl);
   launch_split_samples(static_cast<const float2*>(y), density, P->M, P->C, P->spanel.as<__half>(),
-                       P->norm_parts.as<double>(), kNormParts, st, s);
+                       P->norm_parts.as<double>(), kNormParts, st, s, pdl);
   InterpOut o;
   o.c64 = P->grid.as<float2>();
   o.rows = grid_cells(P);
@@ -1245,8 +1258,8 @@ static tsn_status adjoint_entry(tsn_plan* plan, const void* y, const void* smaps
     if (reference && !plan->view_ref[TSN_VIEW_GT].present)
       fail(TSN_ERR_ARG, "the reference operator needs a plan built with TSN_FLAG_REFERENCE_STEPS");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    enqueue_adjoint_grid(plan, y, nullptr, s, 1, reference);
-    const FftArgs f = fft_args(plan, smaps);
+    const FftArgs f = fft_args(plan, smaps, 1, direct_pdl(s));
+    enqueue_adjoint_grid(plan, y, nullptr, s, 1, reference, f.pdl);
     inv_to_lines(plan, f, plan->grid.as<float2>(), s);
     launch_inv_rows(f, plan->z1.as<float2>(), static_cast<float2*>(x), 0, nullptr, nullptr, nullptr, nullptr,
                     plan->state.as<CgState>(), 0, 1.0f, 0.f, s);
@@ -1289,7 +1302,7 @@ tsn_status tsn_rdot(tsn_plan* plan, const void* a, const void* b, int64_t n, dou
     if (n < 0) fail(TSN_ERR_ARG, "n must be >= 0");
     CUDA_OK(cudaSetDevice(plan->desc.device));
     launch_rdot(static_cast<const float2*>(a), static_cast<const float2*>(b), n, plan->norm_parts.as<double>(), out,
-                reinterpret_cast<cudaStream_t>(stream));
+                reinterpret_cast<cudaStream_t>(stream), direct_pdl(reinterpret_cast<cudaStream_t>(stream)));
     CUDA_OK(cudaGetLastError());
     return TSN_OK;
   } catch (const std::exception& e) {
@@ -1308,7 +1321,7 @@ tsn_status tsn_cg_step(tsn_plan* plan, int64_t n, const double* rho, const doubl
     launch_cg_step(n, plan->adj_parts.as<double>(), rho, gamma, static_cast<const float2*>(x),
                    static_cast<const float2*>(p), static_cast<const float2*>(r), static_cast<const float2*>(q),
                    static_cast<float2*>(x_out), static_cast<float2*>(r_out), static_cast<float2*>(p_out), rho_out,
-                   p_norm_parts, reinterpret_cast<cudaStream_t>(stream));
+                   p_norm_parts, reinterpret_cast<cudaStream_t>(stream), direct_pdl(reinterpret_cast<cudaStream_t>(stream)));
     CUDA_OK(cudaGetLastError());
     return TSN_OK;
   } catch (const std::exception& e) {
@@ -1329,7 +1342,7 @@ tsn_status tsn_cg_adjoint_step(tsn_plan* plan, int64_t n, const double* rho, con
                            static_cast<float2*>(rb), static_cast<float2*>(pb), static_cast<const float2*>(p),
                            static_cast<const float2*>(q), static_cast<const float2*>(r_next),
                            static_cast<const float2*>(xb), static_cast<float2*>(qb), qb_norm_parts,
-                           reinterpret_cast<cudaStream_t>(stream));
+                           reinterpret_cast<cudaStream_t>(stream), direct_pdl(reinterpret_cast<cudaStream_t>(stream)));
     CUDA_OK(cudaGetLastError());
     return TSN_OK;
   } catch (const std::exception& e) {
@@ -1348,7 +1361,8 @@ tsn_status tsn_cg_adjoint_finish(tsn_plan* plan, int64_t n, int32_t coils, void*
     launch_cg_adjoint_finish(n, coils, static_cast<float2*>(pb), static_cast<const float2*>(mqb),
                              static_cast<const float2*>(qb), static_cast<const float2*>(coil_images),
                              static_cast<const float2*>(coil_images_bar), static_cast<const float2*>(p),
-                             static_cast<float2*>(sb), reinterpret_cast<cudaStream_t>(stream));
+                             static_cast<float2*>(sb), reinterpret_cast<cudaStream_t>(stream),
+                             direct_pdl(reinterpret_cast<cudaStream_t>(stream)));
     CUDA_OK(cudaGetLastError());
     return TSN_OK;
   } catch (const std::exception& e) {
