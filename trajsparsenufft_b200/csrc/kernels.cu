@@ -545,6 +545,11 @@ __device__ __forceinline__ void cp_async_bytes(void* dst, const void* src, int b
 // together (one image update, one coil combine).
 __host__ __device__ constexpr int cols_coils(int C) { return C == 16 ? 8 : C; }
 
+// k in [gap.x, gap.y)
+__device__ __forceinline__ bool in_gap(int k, int2 gap) {
+  return static_cast<unsigned>(k - gap.x) < static_cast<unsigned>(gap.y - gap.x);
+}
+
 // Row pitch (float2) of coil-map rows staged in shared memory for a coil-fastest reader:
 // 16 bytes off a multiple of 128, so that 8 coils of two neighbouring pixels share no bank.
 __host__ __device__ __forceinline__ int map_pitch(int N) { return (N + 15) / 16 * 16 + 2; }
@@ -697,7 +702,9 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
     }
     // line i0 = (slab, row): z1 [slab][q][row][c] (one slab for images)
     float2* dst = z1 + (static_cast<size_t>(i0 / N) * G * N + i0 % N) * C + c;
-    F::last(buf, tid, [&](int, int, int k, float2 v) { dst[static_cast<size_t>(k) * N * C] = v; });
+    F::last(buf, tid, [&](int, int, int k, float2 v) {
+      if (!in_gap(k, f.axis_gap)) dst[static_cast<size_t>(k) * N * C] = v;
+    });
   }
 }
 
@@ -716,6 +723,8 @@ fwd_cols_kernel(FftArgs f, const float2* __restrict__ z1, __half* __restrict__ p
   pdl_trigger();
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+    const int2 gap = f.cell_gap ? f.cell_gap[q1] : make_int2(0, 0);
+    if (f.dims == 3 && gap.y - gap.x >= G) continue;  // images: the loads do not wait for the gap's
     if (it != blockIdx.x) __syncthreads();
     const float2* src = z1 + static_cast<size_t>(q1) * N * C + c;
     F::first(buf, f.tw, threadIdx.x, [&](int n) {
@@ -730,6 +739,7 @@ fwd_cols_kernel(FftArgs f, const float2* __restrict__ z1, __half* __restrict__ p
     }
     uint32_t* dst = reinterpret_cast<uint32_t*>(panel + static_cast<size_t>(q1) * G * 4 * C) + c;
     F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+      if (in_gap(k, gap)) return;
       uint32_t hw, rw;
       split_hi_res2(v.x, v.y, hw, rw);
       dst[k * 2 * C] = hw;
@@ -753,6 +763,8 @@ fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1, float2* __restrict__ z2
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
     const int q2 = t / N, i0 = t - q2 * N;
+    const int2 gap = f.line_gap ? f.line_gap[q2] : make_int2(0, 0);
+    if (gap.y - gap.x >= G || in_gap(q2, f.axis_gap)) continue;
     if (it != blockIdx.x) __syncthreads();
     const float2* src = z1 + (static_cast<size_t>(i0) * G + q2) * N * C + c;
     F::first(buf, f.tw, threadIdx.x, [&](int n) {
@@ -766,7 +778,9 @@ fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1, float2* __restrict__ z2
       __syncthreads();
     }
     float2* dst = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
-    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) { dst[static_cast<size_t>(k) * N * C] = v; });
+    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+      if (!in_gap(k, gap)) dst[static_cast<size_t>(k) * N * C] = v;
+    });
   }
 }
 
@@ -817,9 +831,15 @@ inv_cols_kernel(FftArgs f, const float2* __restrict__ grid, float2* __restrict__
   pdl_wait();
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+    // images read the unused cells' zeros: a load of the gap ahead of the line's own costs more
+    const int2 gap = f.dims == 3 && f.cell_gap ? f.cell_gap[q1] : make_int2(0, 0);
+    // a line that the next stage takes as zero (q1 = q2 G + q1 of volumes)
+    if (f.dims == 3 ? (f.line_gap && in_gap(q1 % G, f.line_gap[q1 / G])) || in_gap(q1 / G, f.axis_gap)
+                    : in_gap(q1, f.axis_gap))
+      continue;
     if (it != blockIdx.x) __syncthreads();
     const float2* src = grid + static_cast<size_t>(q1) * G * C + c;
-    F::first(buf, f.tw, threadIdx.x, [&](int n) { return src[n * C]; });
+    F::first(buf, f.tw, threadIdx.x, [&](int n) { return in_gap(n, gap) ? make_float2(0.f, 0.f) : src[n * C]; });
     __syncthreads();
     if constexpr (F::R3 > 1) {
       F::middle(buf, f.tw, threadIdx.x);
@@ -849,9 +869,13 @@ inv_mid_kernel(FftArgs f, const float2* __restrict__ z2, float2* __restrict__ z1
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
     const int q2 = t / N, i0 = t - q2 * N;
+    if (in_gap(q2, f.axis_gap)) continue;
+    const int2 gap = f.line_gap ? f.line_gap[q2] : make_int2(0, 0);
     if (it != blockIdx.x) __syncthreads();
     const float2* src = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
-    F::first(buf, f.tw, threadIdx.x, [&](int n) { return src[static_cast<size_t>(n) * N * C]; });
+    F::first(buf, f.tw, threadIdx.x, [&](int n) {
+      return in_gap(n, gap) ? make_float2(0.f, 0.f) : src[static_cast<size_t>(n) * N * C];
+    });
     __syncthreads();
     if constexpr (F::R3 > 1) {
       F::middle(buf, f.tw, threadIdx.x);
@@ -922,7 +946,9 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
       issue(i0, 3);
     }
     const float2* src = w1 + static_cast<size_t>(i0) * C + c;
-    F::first(buf, f.tw, tid, [&](int n) { return src[static_cast<size_t>(n) * lines * C]; });
+    F::first(buf, f.tw, tid, [&](int n) {
+      return in_gap(n, f.axis_gap) ? make_float2(0.f, 0.f) : src[static_cast<size_t>(n) * lines * C];
+    });
     __syncthreads();
     if constexpr (F::R3 > 1) {
       F::middle(buf, f.tw, tid);

@@ -110,6 +110,13 @@ struct FftArgs {
   bool pdl = false;                     // launch with programmatic dependent launch (direct calls)
   bool maps_early = true;               // forward rows may read the coil maps ahead of pdl_wait: a kernel of
                                         // this call has already waited for the caller's work
+  // Grid cells that no sample of the plan touches: neither written on the way to the
+  // interpolation nor read (zero) on the way back. Trajectories fill a disc or a ball of the
+  // grid, so a fifth of a 2D grid and half of a 3D grid is such corner. Null / empty: none.
+  // The FFT endpoints, whose callers own the whole grid, take none.
+  const int2* cell_gap = nullptr;       // per grid line (gcols): cells [x, y) along the first axis
+  const int2* line_gap = nullptr;       // volumes, per q2: grid lines q1 in [x, y), wholly unused
+  int2 axis_gap = {0, 0};               // last axis (q1 of images, q2 of volumes), wholly unused
   // image lines along the last axis (items of the row stages)
   __host__ __device__ int lines() const { return dims == 3 ? N * N : N; }
   // pixels (voxels) of one image

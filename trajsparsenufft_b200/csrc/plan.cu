@@ -115,6 +115,11 @@ struct tsn_plan {
   int64_t M = 0;
   DevView view[2];
   DeviceBuffer scaling, tw, z1, z2, panel, spanel, grid, r, p, ap, rhs, parts_pap, parts_rr, norm_parts, state;
+  // grid cells that some view gathers or writes (host, while the plan is built), and the gaps
+  // between them (FftArgs::cell_gap, line_gap, axis_gap)
+  std::vector<uint8_t> used;
+  DeviceBuffer cell_gap, line_gap;
+  int2 axis_gap = {0, 0};
   DeviceBuffer adj_parts;  // 5 x 296 FP64 partials of the reverse-mode CG step
   tsn_plan_info info{};
   std::map<GraphKey, cudaGraphExec_t> graphs;
@@ -419,6 +424,7 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
   // persistent warps: contiguous runs of items with about the same number of tiles each;
   // records are stored in that stream order so each warp reads one contiguous range
   const int rowh = 4 * P->C, lanes = gather_lanes(rowh);
+  P->used.resize(static_cast<size_t>(grid_cells(P)), 0);
   std::vector<uint8_t> records(static_cast<size_t>(tiles) * rec, 0);
   d.item_ends.clear();
   int64_t pos = 0;
@@ -432,6 +438,7 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
           const int col = gather_column(rowh, q, j);
           int64_t c = h.tile_col_ids[static_cast<size_t>(t) * kKTile + col];
           if (cols_are_cells) c = to_internal(P, c);
+          if (cols_are_cells && ((live >> col) & 1u)) P->used[static_cast<size_t>(c)] = 1;
           offsets[q * lanes + j] = ((live >> col) & 1u) ? static_cast<uint32_t>(c * rowh * 2) : kGatherDead;
         }
       std::memcpy(r, offsets, sizeof offsets);
@@ -444,9 +451,12 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
       }
       RecordInfo info;
       info.flags = (t == it.t0 ? kRecFirst : 0) | (t + 1 == it.t1 ? kRecLast : 0);
-      for (int s = 0; s < kMTile; ++s)
-        if (h.group_row_ids[static_cast<size_t>(it.group) * kMTile + s] >= 0)
-          info.flags |= static_cast<int32_t>(1u << (kRecLiveShift + s));
+      for (int s = 0; s < kMTile; ++s) {
+        const int32_t v = h.group_row_ids[static_cast<size_t>(it.group) * kMTile + s];
+        if (v < 0) continue;
+        info.flags |= static_cast<int32_t>(1u << (kRecLiveShift + s));
+        if (rows_are_cells) P->used[static_cast<size_t>(to_internal(P, v))] = 1;
+      }
       info.split = it.split;
       info.first_slot = it.first_slot;
       info.chunk = it.chunk | (it.nchunks << 16);
@@ -489,6 +499,41 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
   P->info.active_rows[which] = h.active_rows;
   P->info.nnz[which] = h.nnz;
   P->info.pack_bytes[which] = static_cast<int64_t>(records.size());
+}
+
+// Longest run [x, y) of i in [0, n) with !used(i).
+template <class Used>
+int2 longest_gap(int n, Used used) {
+  int2 best = make_int2(0, 0);
+  for (int i = 0, start = 0; i <= n; ++i) {
+    if (i < n && !used(i)) continue;
+    if (i - start > best.y - best.x) best = make_int2(start, i);
+    start = i + 1;
+  }
+  return best;
+}
+
+// The unused runs of the grid, from P->used (every view uploaded): cells of each grid line,
+// and lines and planes that are unused as a whole.
+void upload_gaps(tsn_plan* P) {
+  const int G = P->G;
+  const int64_t lines = grid_cells(P) / G;
+  std::vector<int2> cells(static_cast<size_t>(lines));
+  for (int64_t l = 0; l < lines; ++l) {
+    const uint8_t* u = P->used.data() + l * G;
+    cells[l] = longest_gap(G, [&](int i) { return u[i] != 0; });
+  }
+  auto whole = [&](int64_t l) { return cells[l].y - cells[l].x == G; };
+  if (P->dims == 3) {
+    std::vector<int2> rows(static_cast<size_t>(G));
+    for (int64_t q2 = 0; q2 < G; ++q2) rows[q2] = longest_gap(G, [&](int q1) { return !whole(q2 * G + q1); });
+    P->axis_gap = longest_gap(G, [&](int q2) { return rows[q2].y - rows[q2].x < G; });
+    P->line_gap.upload(rows);
+  } else {
+    P->axis_gap = longest_gap(G, [&](int q1) { return !whole(q1); });
+  }
+  P->cell_gap.upload(cells);
+  P->used = std::vector<uint8_t>();
 }
 
 void check_desc(const tsn_plan_desc* d) {
@@ -587,8 +632,15 @@ bool direct_pdl(cudaStream_t s) {
   return st == cudaStreamCaptureStatusNone;
 }
 
-FftArgs fft_args(const tsn_plan* P, const void* smaps, int share = 1, bool pdl = false) {
+// gaps: leave out the grid cells that no sample touches (everything but the FFT endpoints, whose
+// callers own the whole grid)
+FftArgs fft_args(const tsn_plan* P, const void* smaps, int share = 1, bool pdl = false, bool gaps = true) {
   FftArgs f;
+  if (gaps) {
+    f.cell_gap = P->cell_gap.as<int2>();
+    f.line_gap = P->line_gap.as<int2>();
+    f.axis_gap = P->axis_gap;
+  }
   f.pdl = pdl;
   f.share = share;
   f.N = P->N;
@@ -824,6 +876,7 @@ tsn_status tsn_plan_create_from_pack(const char* fwd_real, const char* fwd_imag,
     P->use_tc = choose_tc(desc, P->ncomp, P->C);
     if (fwd_real) upload_view(P.get(), TSN_VIEW_G, hv[0], false, true);
     if (adj_real) upload_view(P.get(), TSN_VIEW_GT, hv[1], true, false);
+    upload_gaps(P.get());
     allocate_workspaces(P.get());
     setup_tc(P.get());
     P->info.samples = P->M;
@@ -902,7 +955,8 @@ tsn_status tsn_plan_create_from_trajectory(const float* traj, int64_t m, const t
       hv[0] = HostView();
       upload_view(P.get(), TSN_VIEW_GT, hv[1], true, false);
       hv[1] = HostView();
-      allocate_workspaces(P.get());
+      upload_gaps(P.get());
+    allocate_workspaces(P.get());
       setup_tc(P.get());
       P->info.samples = P->M;
       P->info.im_size = P->N;
@@ -967,6 +1021,7 @@ tsn_status tsn_plan_create_from_trajectory(const float* traj, int64_t m, const t
       upload_view(P.get(), TSN_VIEW_GT, hv_ref[1], true, false, &P->view_ref[TSN_VIEW_GT]);
       for (DevView& d : P->view_ref) d.v.sum_components = 1;
     }
+    upload_gaps(P.get());
     allocate_workspaces(P.get());
     setup_tc(P.get());
     P->info.samples = P->M;
@@ -1669,7 +1724,7 @@ tsn_status tsn_fft_forward_panel(tsn_plan* plan, const void* x, const void* smap
     need_aligned({x, smaps, panel_f16});
     need_views(plan, false, false);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const FftArgs f = fft_args(plan, smaps);
+    const FftArgs f = fft_args(plan, smaps, 1, false, false);
     CgState* st = plan->state.as<CgState>();
     const int64_t n = image_pixels(plan) * (smaps ? 1 : plan->C);
     launch_norm_partials(static_cast<const float2*>(x), n, plan->norm_parts.as<double>(), s);
@@ -1695,7 +1750,7 @@ tsn_status tsn_fft_adjoint_image(tsn_plan* plan, const void* grid_c64, const voi
     need_aligned({grid_c64, smaps, x});
     need_views(plan, false, false);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const FftArgs f = fft_args(plan, smaps);
+    const FftArgs f = fft_args(plan, smaps, 1, false, false);
     CgState* st = plan->state.as<CgState>();
     // unit sample scale for the plain adjoint epilogue (factor = 1 / sigma_y)
     const float one = 1.0f;
