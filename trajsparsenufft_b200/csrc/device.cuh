@@ -128,81 +128,44 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Deterministic block sum of one double per thread (fixed reduction tree), returned to
-// every thread. `scratch` holds 33 doubles.
+// Deterministic block sum of one double per thread (fixed order), returned to every thread.
+// `scratch` holds 32 doubles; it may be reused at once.
 __device__ __forceinline__ double block_sum(double v, double* scratch) {
   v = warp_sum(v);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) scratch[warp] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += scratch[w];
-    scratch[32] = t;
-  }
-  __syncthreads();
-  const double t = scratch[32];
-  __syncthreads();  // scratch may be reused by the caller's next block_sum
-  return t;
-}
-
-// Three deterministic block sums at once (one pass of barriers); `scratch` holds 99 doubles.
-__device__ __forceinline__ double3 block_sum3(double a, double b, double c, double* scratch) {
-  a = warp_sum(a);
-  b = warp_sum(b);
-  c = warp_sum(c);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    scratch[warp] = a;
-    scratch[33 + warp] = b;
-    scratch[66 + warp] = c;
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += scratch[33 * threadIdx.x + w];
-    scratch[33 * threadIdx.x + 32] = t;
-  }
-  __syncthreads();
-  const double3 t = make_double3(scratch[32], scratch[65], scratch[98]);
+  const int nw = (blockDim.x + 31) >> 5;
+  double t = 0.0;
+  for (int w = 0; w < nw; ++w) t += scratch[w];
   __syncthreads();
   return t;
 }
 
-// Four deterministic block sums at once; `scratch` holds 132 doubles.
-__device__ __forceinline__ double4 block_sum4(double a, double b, double c, double d, double* scratch) {
-  a = warp_sum(a);
-  b = warp_sum(b);
-  c = warp_sum(c);
-  d = warp_sum(d);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    scratch[warp] = a;
-    scratch[33 + warp] = b;
-    scratch[66 + warp] = c;
-    scratch[99 + warp] = d;
-  }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += scratch[33 * threadIdx.x + w];
-    scratch[33 * threadIdx.x + 32] = t;
-  }
-  __syncthreads();
-  const double4 t = make_double4(scratch[32], scratch[65], scratch[98], scratch[131]);
-  __syncthreads();
-  return t;
+// Warp sums of four doubles per lane in six exchanges instead of twenty: each halving of the
+// lanes also halves the values a lane keeps. Lanes 0, 8, 16, 24 (and the seven after each)
+// return the sums of a, b, c, d.
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d) {
+  const int lane = threadIdx.x & 31;
+  const bool upper = lane & 16, odd = lane & 8;
+  double k0 = upper ? c : a, k1 = upper ? d : b;
+  k0 += __shfl_xor_sync(0xFFFFFFFFu, upper ? a : c, 16);
+  k1 += __shfl_xor_sync(0xFFFFFFFFu, upper ? b : d, 16);
+  double k = odd ? k1 : k0;
+  k += __shfl_xor_sync(0xFFFFFFFFu, odd ? k0 : k1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(0xFFFFFFFFu, k, o);
+  return k;
 }
 
-// Power-of-two scale bringing rms to ~target (FP16 rounding commutes with it).
+// Power-of-two scale bringing rms to ~target (FP16 rounding commutes with it): the nearest
+// power (on the logarithm) of target / rms, from the exponent of 2 (target / rms)^2. Every CTA
+// of a row stage waits for it, so no square root, logarithm or power is taken.
 __device__ __forceinline__ float pow2_scale(double sum_sq, double count, float target) {
-  const double rms = sqrt(sum_sq / count);
-  if (!(rms > 0.0) || !isfinite(rms)) return 1.0f;
-  const double e = rint(log2(static_cast<double>(target) / rms));
-  return static_cast<float>(exp2(fmin(fmax(e, -100.0), 100.0)));
+  if (!(sum_sq > 0.0) || !isfinite(sum_sq)) return 1.0f;
+  const double q = 2.0 * static_cast<double>(target) * target * count / sum_sq;
+  const int e = (((__double2hiint(q) >> 20) & 0x7FF) - 1023) >> 1;  // floor(log2(q) / 2)
+  return __int_as_float((min(max(e, -100), 100) + 127) << 23);
 }
 
 }  // namespace dev

@@ -488,14 +488,18 @@ void launch_interp(const InterpView& v, const __half* panel, int rowh, bool spli
 // ------------------------------------------------------------------------------------------
 // Reductions
 // ------------------------------------------------------------------------------------------
+// n is even and v 16-byte aligned (images and coil k-space of 4 k coils)
 __global__ void norm_partials_kernel(const float2* __restrict__ v, int64_t n, double* __restrict__ part) {
-  __shared__ double scratch[33];
+  __shared__ double scratch[32];
   pdl_wait();
+  const float4* v4 = reinterpret_cast<const float4*>(v);
   double acc = 0.0;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+#pragma unroll 4
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 2;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const float2 x = v[i];
-    acc += static_cast<double>(x.x) * x.x + static_cast<double>(x.y) * x.y;
+    const float4 x = v4[i];
+    acc += static_cast<double>(x.x) * x.x + static_cast<double>(x.y) * x.y + static_cast<double>(x.z) * x.z +
+           static_cast<double>(x.w) * x.w;
   }
   const double t = block_sum(acc, scratch);
   if (threadIdx.x == 0) part[blockIdx.x] = t;
@@ -512,16 +516,30 @@ __device__ __forceinline__ double sum_partials(const double* part, int nparts, d
   return block_sum(a, scratch);
 }
 
-// Sums of four partial sections [nparts] spaced `stride` apart, as sum_partials does each.
+// Sums of four partial sections [nparts] spaced `stride` apart, in a fixed order. Each warp
+// takes a strided piece of one section, so that a section's sum costs one tree of exchanges
+// and not one per warp and section. `scratch` holds 32 doubles.
 __device__ __forceinline__ double4 sum_partials4(const double* part, int nparts, int64_t stride, double* scratch) {
-  double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-    a += part[i];
-    b += part[stride + i];
-    c += part[2 * stride + i];
-    d += part[3 * stride + i];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int pieces = nw > 4 ? nw / 4 : 1;
+  for (int t = warp; t < 4 * pieces; t += nw) {
+    const double* sec = part + (t & 3) * stride;
+    double a = 0.0;
+#pragma unroll 4
+    for (int i = (t >> 2) * 32 + lane; i < nparts; i += 32 * pieces) a += sec[i];
+    a = warp_sum(a);
+    if (lane == 0) scratch[t] = a;
   }
-  return block_sum4(a, b, c, d, scratch);
+  __syncthreads();
+  double4 r = make_double4(0.0, 0.0, 0.0, 0.0);
+  for (int k = 0; k < pieces; ++k) {
+    r.x += scratch[4 * k];
+    r.y += scratch[4 * k + 1];
+    r.z += scratch[4 * k + 2];
+    r.w += scratch[4 * k + 3];
+  }
+  __syncthreads();
+  return r;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -789,8 +807,21 @@ fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1, float2* __restrict__ z2
 __global__ void split_samples_kernel(const float2* __restrict__ y, const float* __restrict__ density, int64_t m,
                                      int C, __half* __restrict__ panel, const double* __restrict__ parts, int nparts,
                                      CgState* __restrict__ st) {
-  __shared__ double red[33];
+  __shared__ double red[32];
+  const int chunks = C / 4;
+  const int64_t n = m * chunks, step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  float2 val[4];
+  float w = 1.f;
+  auto fetch = [&]() {
+    const int64_t row = i / chunks;
+    const int q = static_cast<int>(i - row * chunks);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) val[k] = y[static_cast<size_t>(4 * q + k) * m + row];
+    if (density) w = density[row];
+  };
   pdl_wait();
+  if (i < n) fetch();  // the first values travel while the scale is reduced
   const double total = sum_partials(parts, nparts, red);
   const float sigma = pow2_scale(total, static_cast<double>(m) * C, kPanelTarget);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -799,21 +830,18 @@ __global__ void split_samples_kernel(const float2* __restrict__ y, const float* 
     st->finite_ok = 1;
     st->completed = 0;
   }
-  const int chunks = C / 4;
   uint32_t* pu = reinterpret_cast<uint32_t*>(panel);
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < m * chunks;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  while (i < n) {
     const int64_t row = i / chunks;
     const int q = static_cast<int>(i - row * chunks);
-    const float w = sigma * (density ? density[row] : 1.0f);
+    const float ws = sigma * w;
     uint32_t hi[4], res[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 val = y[static_cast<size_t>(4 * q + k) * m + row];
-      split_hi_res2(val.x * w, val.y * w, hi[k], res[k]);
-    }
+    for (int k = 0; k < 4; ++k) split_hi_res2(val[k].x * ws, val[k].y * ws, hi[k], res[k]);
     *reinterpret_cast<uint4*>(pu + row * 2 * C + 4 * q) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(pu + row * 2 * C + C + 4 * q) = make_uint4(res[0], res[1], res[2], res[3]);
+    i += step;
+    if (i < n) fetch();
   }
 }
 
@@ -1020,12 +1048,13 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
       }
     }
     if (mode == 2 && r) {
-      const double4 t = block_sum4(dot, dot_r, dot_a, dot_rr, red);
-      if (tid == 0) {
-        parts[i0] = t.x;
-        parts[lines + i0] = t.y;
-        parts[2 * static_cast<int64_t>(lines) + i0] = t.z;
-        parts[3 * static_cast<int64_t>(lines) + i0] = t.w;
+      const double t = warp_sum4(dot, dot_r, dot_a, dot_rr);
+      if ((tid & 7) == 0) red[(tid >> 3 & 3) * 32 + (tid >> 5)] = t;
+      __syncthreads();
+      if (tid < 4) {
+        double total = 0.0;
+        for (int w = 0; w < F::THREADS / 32; ++w) total += red[tid * 32 + w];
+        parts[tid * static_cast<int64_t>(lines) + i0] = total;
       }
     } else if (mode != 0) {
       const double t = block_sum(dot, red);
