@@ -274,6 +274,27 @@ struct LineFft {
       }
     }
   }
+  // The last pass in place: output k is left in shared row out_row(k).
+  static __host__ __device__ __forceinline__ void last_in_place(float2* s, int tid) {
+    const int c = tid % C, b0 = tid / C;
+#pragma unroll
+    for (int i = 0; i < ITL; ++i) {
+      const int b = b0 + i * TB;
+      if (NL % TB == 0 || b < NL) {
+        float2* q = s + ((R3 > 1 ? RL * (b / R1) : 0) + (S1 + 1) * (b % R1)) * C + c;
+        float2 v[RL];
+#pragma unroll
+        for (int j = 0; j < RL; ++j) v[j] = q[j * C];
+        Dft<RL, INV>::run(v);
+#pragma unroll
+        for (int j = 0; j < RL; ++j) q[j * C] = v[j];
+      }
+    }
+  }
+  static __host__ __device__ __forceinline__ int out_row(int k) {
+    const int b = k % NL, j = k / NL;
+    return (R3 > 1 ? RL * (b / R1) : 0) + (S1 + 1) * (b % R1) + j;
+  }
   // last-pass butterfly of iteration i of thread tid (its outputs: b + NL j), or -1
   static __host__ __device__ __forceinline__ int last_base(int tid, int i) {
     const int b = tid / C + i * TB;

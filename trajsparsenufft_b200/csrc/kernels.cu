@@ -555,7 +555,15 @@ __device__ __forceinline__ void cp_async_bytes(void* dst, const void* src, int b
 // CTAs per SM that the register cap leaves room for: 1024 threads at 64 registers, and for the
 // row stages, which hold a line's last butterflies and its epilogue, 768 at 80.
 #define TSN_FFT_BOUNDS(T) __launch_bounds__((T), (1024 / (T)) > 0 ? 1024 / (T) : 1)
-#define TSN_ROW_BOUNDS(T) __launch_bounds__((T), (768 / (T)) > 0 ? 768 / (T) : 1)
+#define TSN_ROW_BOUNDS(T) __launch_bounds__((T), (T) <= 256 ? 768 / (T) : (T) <= 640 ? 2 : 1)
+
+// Lines of more than 256 threads (12 and 16 coils, large grids) leave the last inverse butterflies
+// in shared memory instead
+// of holding them in registers while the region changes hands: two CTAs of 480-640 threads
+// then stay resident per SM, where one CTA per SM took three waves for 320 lines. The smaller
+// lines hold them: their images are then read without bank conflicts. 320^2 x 12 coils: 21.2 -> 15 us.
+template <class F>
+__host__ __device__ constexpr bool rows_in_place() { return F::THREADS > 256; }
 
 // Coils per CTA of the column and middle stages. 16 coils go in two CTAs of 8: a 64-byte run
 // per row is still whole sectors, and the smaller CTA halves shared memory, so that several
@@ -919,7 +927,8 @@ inv_mid_kernel(FftArgs f, const float2* __restrict__ z2, float2* __restrict__ z1
 }
 
 // Inverse rows + crop + deapodization + SENSE coil combine (+ CG epilogues).
-// Shared memory: FFT rows [G + R1][C], then the coil images [N][C+1] in their place |
+// Shared memory: FFT rows [G + R1][C], then (rows_in_place: permuted) the coil images [N][C+1]
+// in their place |
 // (epi_smem) the epilogue inputs of the row, copied while the line is transformed: maps
 // [C][N] (with smaps), p row [N] (modes 2, 3, 5), r or b row [N] (modes 2 with r, 3), scaling
 // row [N] float. Without epi_smem the epilogue reads them from global memory.
@@ -982,20 +991,25 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
       F::middle(buf, f.tw, tid);
       __syncthreads();
     }
-    float2 v[F::ITL][F::RL];
-    F::last(buf, tid, [&](int i, int j, int, float2 val) { v[i][j] = val; });
-    cp_async_wait<0>();
-    __syncthreads();  // the FFT rows are read: the region becomes the coil images
-    float2* img_s = buf;  // [N][C+1]
+    float2* img_s = buf;
+    if constexpr (rows_in_place<F>()) {
+      F::last_in_place(buf, tid);
+      cp_async_wait<0>();
+    } else {
+      float2 v[F::ITL][F::RL];
+      F::last(buf, tid, [&](int i, int j, int, float2 val) { v[i][j] = val; });
+      cp_async_wait<0>();
+      __syncthreads();  // the FFT rows are read: the region becomes the coil images [N][C+1]
 #pragma unroll
-    for (int i = 0; i < F::ITL; ++i) {
-      const int b = F::last_base(tid, i);
-      if (b < 0) continue;
+      for (int i = 0; i < F::ITL; ++i) {
+        const int b = F::last_base(tid, i);
+        if (b < 0) continue;
 #pragma unroll
-      for (int j = 0; j < F::RL; ++j) {
-        int i1 = b + F::NL * j + f.shift;
-        if (i1 >= G) i1 -= G;
-        if (i1 < N) img_s[i1 * (C + 1) + c] = v[i][j];
+        for (int j = 0; j < F::RL; ++j) {
+          int i1 = b + F::NL * j + f.shift;
+          if (i1 >= G) i1 -= G;
+          if (i1 < N) img_s[i1 * (C + 1) + c] = v[i][j];
+        }
       }
     }
     __syncthreads();
@@ -1003,7 +1017,8 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
     for (int i1 = tid; i1 < N; i1 += blockDim.x) {
       const size_t pix = static_cast<size_t>(i0) * N + i1;
       const float d = (epi_smem ? escale[i1] : f.scaling[pix]) * factor;
-      const float2* img = img_s + i1 * (C + 1);
+      const int k = i1 >= f.shift ? i1 - f.shift : i1 - f.shift + G;  // the pixel's grid position
+      const float2* img = img_s + (rows_in_place<F>() ? F::out_row(k) * C : i1 * (C + 1));
       if (!f.smaps) {  // coil images out [C][N][N]
 #pragma unroll
         for (int cc = 0; cc < C; ++cc) out[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
@@ -1259,7 +1274,8 @@ void launch_inv_rows(const FftArgs& f, const float2* w1, float2* out, int mode, 
                      double* partials, CgState* st, int iter, float inv_scale2, float lambda_scaled, cudaStream_t s) {
   TSN_G_SWITCH(f.G, TSN_FFT_C(f.C, {
     const size_t img = sizeof(float2) * static_cast<size_t>(f.N) * (CC + 1);
-    const size_t region = align16(std::max(fft_rows_bytes<GG, CC>(), img));
+    const size_t region =
+        rows_in_place<LineFft<GG, CC, true>>() ? fft_rows_bytes<GG, CC>() : align16(std::max(fft_rows_bytes<GG, CC>(), img));
     const int rows = (f.smaps ? CC : 0) + (mode >= 2 ? 1 : 0) + ((mode == 2 && r) || mode == 3 ? 1 : 0);
     const size_t epi = (sizeof(float2) * rows + sizeof(float)) * static_cast<size_t>(f.N);
     const int epi_smem = region + epi <= kFftStageSmem ? 1 : 0;
