@@ -557,11 +557,11 @@ __device__ __forceinline__ void cp_async_bytes(void* dst, const void* src, int b
 #define TSN_FFT_BOUNDS(T) __launch_bounds__((T), (1024 / (T)) > 0 ? 1024 / (T) : 1)
 #define TSN_ROW_BOUNDS(T) __launch_bounds__((T), (T) <= 256 ? 768 / (T) : (T) <= 640 ? 2 : 1)
 
-// Lines of more than 256 threads (12 and 16 coils, large grids) leave the last inverse butterflies
-// in shared memory instead
-// of holding them in registers while the region changes hands: two CTAs of 480-640 threads
-// then stay resident per SM, where one CTA per SM took three waves for 320 lines. The smaller
-// lines hold them: their images are then read without bank conflicts. 320^2 x 12 coils: 21.2 -> 15 us.
+// Lines of more than 256 threads (12 and 16 coils, large grids) leave the last inverse
+// butterflies in shared memory instead of holding them in registers while the region changes
+// hands: two CTAs of 480-640 threads then stay resident per SM, where one CTA per SM took three
+// waves for 320 lines (320^2 x 12 coils normal operator 116 -> 109 us). The smaller lines hold
+// them: their images are then read without bank conflicts.
 template <class F>
 __host__ __device__ constexpr bool rows_in_place() { return F::THREADS > 256; }
 
@@ -620,8 +620,9 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
   __shared__ double red[132];
   const int tid = threadIdx.x, c = tid % C;
   // part 1: rows no kernel of a solve writes (coil maps, deapodization); part 2: the rest
-  auto issue = [&](int i0, int part) {
-    const size_t off = static_cast<size_t>(i0) * N;
+  const int i0 = blockIdx.x;
+  const size_t off = static_cast<size_t>(i0) * N;
+  auto issue = [&](int part) {
     if (part & 1) {
       cp_async_bytes(srow, f.scaling + off, N * 4);
       if (stage_maps)
@@ -639,10 +640,10 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
     }
     cp_async_commit();
   };
-  if (f.maps_early && blockIdx.x < lines) issue(blockIdx.x, 1);
+  if (f.maps_early) issue(1);
   pdl_wait();
-  if (!f.maps_early && blockIdx.x < lines) issue(blockIdx.x, 1);
-  if (blockIdx.x < lines) issue(blockIdx.x, 2);
+  if (!f.maps_early) issue(1);
+  issue(2);
   double total, alpha = 0.0, rho_prev = 0.0;
   if (mode == 4) {  // finish iteration iter-1 (the cg_update scalars)
     const double4 s3 = sum_partials4(parts, nparts, lines, red);
@@ -685,53 +686,46 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
   }
   const float scl = sigma / f.gs();
   const bool sense = f.smaps || mode >= 1;
-  for (int i0 = blockIdx.x; i0 < lines; i0 += gridDim.x) {
-    if (i0 != blockIdx.x) {
-      __syncthreads();  // the previous line's shared rows are read
-      issue(i0, 3);
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int i = tid; i < N; i += F::THREADS) {
+    const float d = srow[i] * scl;
+    if (!sense) {
+      row0[i].x = d;
+      continue;
     }
-    const size_t off = static_cast<size_t>(i0) * N;
-    cp_async_wait<0>();
-    __syncthreads();
-    for (int i = tid; i < N; i += F::THREADS) {
-      const float d = srow[i] * scl;
-      if (!sense) {
-        row0[i].x = d;
-        continue;
+    float2 v = row0[i];
+    if (has_beta) {
+      const float2 pv = row1[i];
+      if (mode == 4) {  // x += alpha p, r -= alpha Ap (the previous iteration's update)
+        v = axpy64(-alpha, row2[i], v);
+        r[off + i] = v;
+        xs[off + i] = axpy64(alpha, pv, row3[i]);
       }
-      float2 v = row0[i];
-      if (has_beta) {
-        const float2 pv = row1[i];
-        if (mode == 4) {  // x += alpha p, r -= alpha Ap (the previous iteration's update)
-          v = axpy64(-alpha, row2[i], v);
-          r[off + i] = v;
-          xs[off + i] = axpy64(alpha, pv, row3[i]);
-        }
-        v = axpy64(beta, pv, v);
-      }
-      if (mode >= 1) p[off + i] = v;
-      row0[i] = cscale(v, d);
+      v = axpy64(beta, pv, v);
     }
-    __syncthreads();
-    const float2* msrc = stage_maps ? maps_s + c * pitch : (f.smaps ? f.smaps : x) + static_cast<size_t>(c) * pix + off;
-    F::first(buf, f.tw, tid, [&](int n) {
-      int i1 = n + f.shift;
-      if (i1 >= G) i1 -= G;
-      if (i1 >= N) return make_float2(0.f, 0.f);
-      const float2 w = row0[i1];
-      return sense ? cmul(w, msrc[i1]) : cscale(msrc[i1], w.x);
-    });
-    __syncthreads();
-    if constexpr (F::R3 > 1) {
-      F::middle(buf, f.tw, tid);
-      __syncthreads();
-    }
-    // line i0 = (slab, row): z1 [slab][q][row][c] (one slab for images)
-    float2* dst = z1 + (static_cast<size_t>(i0 / N) * G * N + i0 % N) * C + c;
-    F::last(buf, tid, [&](int, int, int k, float2 v) {
-      if (!in_gap(k, f.axis_gap)) dst[static_cast<size_t>(k) * N * C] = v;
-    });
+    if (mode >= 1) p[off + i] = v;
+    row0[i] = cscale(v, d);
   }
+  __syncthreads();
+  const float2* msrc = stage_maps ? maps_s + c * pitch : (f.smaps ? f.smaps : x) + static_cast<size_t>(c) * pix + off;
+  F::first(buf, f.tw, tid, [&](int n) {
+    int i1 = n + f.shift;
+    if (i1 >= G) i1 -= G;
+    if (i1 >= N) return make_float2(0.f, 0.f);
+    const float2 w = row0[i1];
+    return sense ? cmul(w, msrc[i1]) : cscale(msrc[i1], w.x);
+  });
+  __syncthreads();
+  if constexpr (F::R3 > 1) {
+    F::middle(buf, f.tw, tid);
+    __syncthreads();
+  }
+  // line i0 = (slab, row): z1 [slab][q][row][c] (one slab for images)
+  float2* dst = z1 + (static_cast<size_t>(i0 / N) * G * N + i0 % N) * C + c;
+  F::last(buf, tid, [&](int, int, int k, float2 v) {
+    if (!in_gap(k, f.axis_gap)) dst[static_cast<size_t>(k) * N * C] = v;
+  });
 }
 
 // Forward columns (y-stage): z1[q1][*][c] -> panel rows q1*G + q0, FP16 hi | res.
@@ -744,34 +738,32 @@ fwd_cols_kernel(FftArgs f, const float2* __restrict__ z1, __half* __restrict__ p
   using F = LineFft<G, CC, false>;
   extern __shared__ __align__(16) uint8_t sm[];
   float2* buf = reinterpret_cast<float2*>(sm);
-  const int N = f.N, items = f.gcols() * GROUPS;
+  const int N = f.N;
   pdl_wait();
   pdl_trigger();
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
-    const int2 gap = f.cell_gap ? f.cell_gap[q1] : make_int2(0, 0);
-    if (f.dims == 3 && gap.y - gap.x >= G) continue;  // images: the loads do not wait for the gap's
-    if (it != blockIdx.x) __syncthreads();
-    const float2* src = z1 + static_cast<size_t>(q1) * N * C + c;
-    F::first(buf, f.tw, threadIdx.x, [&](int n) {
-      int i0 = n + f.shift;
-      if (i0 >= G) i0 -= G;
-      return i0 < N ? src[i0 * C] : make_float2(0.f, 0.f);
-    });
+  const int it = blockIdx.x;
+  const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+  const int2 gap = f.cell_gap ? f.cell_gap[q1] : make_int2(0, 0);
+  if (f.dims == 3 && gap.y - gap.x >= G) return;  // images: the loads do not wait for the gap's
+  const float2* src = z1 + static_cast<size_t>(q1) * N * C + c;
+  F::first(buf, f.tw, threadIdx.x, [&](int n) {
+    int i0 = n + f.shift;
+    if (i0 >= G) i0 -= G;
+    return i0 < N ? src[i0 * C] : make_float2(0.f, 0.f);
+  });
+  __syncthreads();
+  if constexpr (F::R3 > 1) {
+    F::middle(buf, f.tw, threadIdx.x);
     __syncthreads();
-    if constexpr (F::R3 > 1) {
-      F::middle(buf, f.tw, threadIdx.x);
-      __syncthreads();
-    }
-    uint32_t* dst = reinterpret_cast<uint32_t*>(panel + static_cast<size_t>(q1) * G * 4 * C) + c;
-    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
-      if (in_gap(k, gap)) return;
-      uint32_t hw, rw;
-      split_hi_res2(v.x, v.y, hw, rw);
-      dst[k * 2 * C] = hw;
-      dst[k * 2 * C + C] = rw;
-    });
   }
+  uint32_t* dst = reinterpret_cast<uint32_t*>(panel + static_cast<size_t>(q1) * G * 4 * C) + c;
+  F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+    if (in_gap(k, gap)) return;
+    uint32_t hw, rw;
+    split_hi_res2(v.x, v.y, hw, rw);
+    dst[k * 2 * C] = hw;
+    dst[k * 2 * C + C] = rw;
+  });
 }
 
 // Forward middle axis of a volume: z1[i0][q2][i1][c] -> z2[q2][q1][i0][c]. One item per line
@@ -784,30 +776,28 @@ fwd_mid_kernel(FftArgs f, const float2* __restrict__ z1, float2* __restrict__ z2
   using F = LineFft<G, CC, false>;
   extern __shared__ __align__(16) uint8_t sm[];
   float2* buf = reinterpret_cast<float2*>(sm);
-  const int N = f.N, items = N * G * GROUPS;
+  const int N = f.N;
   pdl_wait();
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
-    const int q2 = t / N, i0 = t - q2 * N;
-    const int2 gap = f.line_gap ? f.line_gap[q2] : make_int2(0, 0);
-    if (gap.y - gap.x >= G || in_gap(q2, f.axis_gap)) continue;
-    if (it != blockIdx.x) __syncthreads();
-    const float2* src = z1 + (static_cast<size_t>(i0) * G + q2) * N * C + c;
-    F::first(buf, f.tw, threadIdx.x, [&](int n) {
-      int i1 = n + f.shift;
-      if (i1 >= G) i1 -= G;
-      return i1 < N ? src[i1 * C] : make_float2(0.f, 0.f);
-    });
+  const int it = blockIdx.x;
+  const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+  const int q2 = t / N, i0 = t - q2 * N;
+  const int2 gap = f.line_gap ? f.line_gap[q2] : make_int2(0, 0);
+  if (gap.y - gap.x >= G || in_gap(q2, f.axis_gap)) return;
+  const float2* src = z1 + (static_cast<size_t>(i0) * G + q2) * N * C + c;
+  F::first(buf, f.tw, threadIdx.x, [&](int n) {
+    int i1 = n + f.shift;
+    if (i1 >= G) i1 -= G;
+    return i1 < N ? src[i1 * C] : make_float2(0.f, 0.f);
+  });
+  __syncthreads();
+  if constexpr (F::R3 > 1) {
+    F::middle(buf, f.tw, threadIdx.x);
     __syncthreads();
-    if constexpr (F::R3 > 1) {
-      F::middle(buf, f.tw, threadIdx.x);
-      __syncthreads();
-    }
-    float2* dst = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
-    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
-      if (!in_gap(k, gap)) dst[static_cast<size_t>(k) * N * C] = v;
-    });
   }
+  float2* dst = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
+  F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+    if (!in_gap(k, gap)) dst[static_cast<size_t>(k) * N * C] = v;
+  });
 }
 
 // Measurement / adjoint input [C][M] -> sample panel [M][4C] with sigma_y and density.
@@ -863,31 +853,29 @@ inv_cols_kernel(FftArgs f, const float2* __restrict__ grid, float2* __restrict__
   using F = LineFft<G, CC, true>;
   extern __shared__ __align__(16) uint8_t sm[];
   float2* buf = reinterpret_cast<float2*>(sm);
-  const int N = f.N, items = f.gcols() * GROUPS;
+  const int N = f.N;
   pdl_wait();
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
-    // images read the unused cells' zeros: a load of the gap ahead of the line's own costs more
-    const int2 gap = f.dims == 3 && f.cell_gap ? f.cell_gap[q1] : make_int2(0, 0);
-    // a line that the next stage takes as zero (q1 = q2 G + q1 of volumes)
-    if (f.dims == 3 ? (f.line_gap && in_gap(q1 % G, f.line_gap[q1 / G])) || in_gap(q1 / G, f.axis_gap)
-                    : in_gap(q1, f.axis_gap))
-      continue;
-    if (it != blockIdx.x) __syncthreads();
-    const float2* src = grid + static_cast<size_t>(q1) * G * C + c;
-    F::first(buf, f.tw, threadIdx.x, [&](int n) { return in_gap(n, gap) ? make_float2(0.f, 0.f) : src[n * C]; });
+  const int it = blockIdx.x;
+  const int q1 = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+  // images read the unused cells' zeros: a load of the gap ahead of the line's own costs more
+  const int2 gap = f.dims == 3 && f.cell_gap ? f.cell_gap[q1] : make_int2(0, 0);
+  // a line that the next stage takes as zero (q1 = q2 G + q1 of volumes)
+  if (f.dims == 3 ? (f.line_gap && in_gap(q1 % G, f.line_gap[q1 / G])) || in_gap(q1 / G, f.axis_gap)
+                  : in_gap(q1, f.axis_gap))
+    return;
+  const float2* src = grid + static_cast<size_t>(q1) * G * C + c;
+  F::first(buf, f.tw, threadIdx.x, [&](int n) { return in_gap(n, gap) ? make_float2(0.f, 0.f) : src[n * C]; });
+  __syncthreads();
+  if constexpr (F::R3 > 1) {
+    F::middle(buf, f.tw, threadIdx.x);
     __syncthreads();
-    if constexpr (F::R3 > 1) {
-      F::middle(buf, f.tw, threadIdx.x);
-      __syncthreads();
-    }
-    float2* dst = w1 + static_cast<size_t>(q1) * N * C + c;
-    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
-      int i0 = k + f.shift;
-      if (i0 >= G) i0 -= G;
-      if (i0 < N) dst[i0 * C] = v;
-    });
   }
+  float2* dst = w1 + static_cast<size_t>(q1) * N * C + c;
+  F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+    int i0 = k + f.shift;
+    if (i0 >= G) i0 -= G;
+    if (i0 < N) dst[i0 * C] = v;
+  });
 }
 
 // Inverse middle axis of a volume: z2[q2][q1][i0][c] -> z1[q2][i0][i1][c], i1 < N (crop).
@@ -900,30 +888,28 @@ inv_mid_kernel(FftArgs f, const float2* __restrict__ z2, float2* __restrict__ z1
   using F = LineFft<G, CC, true>;
   extern __shared__ __align__(16) uint8_t sm[];
   float2* buf = reinterpret_cast<float2*>(sm);
-  const int N = f.N, items = G * N * GROUPS;
+  const int N = f.N;
   pdl_wait();
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
-    const int q2 = t / N, i0 = t - q2 * N;
-    if (in_gap(q2, f.axis_gap)) continue;
-    const int2 gap = f.line_gap ? f.line_gap[q2] : make_int2(0, 0);
-    if (it != blockIdx.x) __syncthreads();
-    const float2* src = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
-    F::first(buf, f.tw, threadIdx.x, [&](int n) {
-      return in_gap(n, gap) ? make_float2(0.f, 0.f) : src[static_cast<size_t>(n) * N * C];
-    });
+  const int it = blockIdx.x;
+  const int t = it / GROUPS, c = it % GROUPS * CC + threadIdx.x % CC;
+  const int q2 = t / N, i0 = t - q2 * N;
+  if (in_gap(q2, f.axis_gap)) return;
+  const int2 gap = f.line_gap ? f.line_gap[q2] : make_int2(0, 0);
+  const float2* src = z2 + (static_cast<size_t>(q2) * G * N + i0) * C + c;
+  F::first(buf, f.tw, threadIdx.x, [&](int n) {
+    return in_gap(n, gap) ? make_float2(0.f, 0.f) : src[static_cast<size_t>(n) * N * C];
+  });
+  __syncthreads();
+  if constexpr (F::R3 > 1) {
+    F::middle(buf, f.tw, threadIdx.x);
     __syncthreads();
-    if constexpr (F::R3 > 1) {
-      F::middle(buf, f.tw, threadIdx.x);
-      __syncthreads();
-    }
-    float2* dst = z1 + static_cast<size_t>(t) * N * C + c;
-    F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
-      int i1 = k + f.shift;
-      if (i1 >= G) i1 -= G;
-      if (i1 < N) dst[i1 * C] = v;
-    });
   }
+  float2* dst = z1 + static_cast<size_t>(t) * N * C + c;
+  F::last(buf, threadIdx.x, [&](int, int, int k, float2 v) {
+    int i1 = k + f.shift;
+    if (i1 >= G) i1 -= G;
+    if (i1 < N) dst[i1 * C] = v;
+  });
 }
 
 // Inverse rows + crop + deapodization + SENSE coil combine (+ CG epilogues).
@@ -956,8 +942,9 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
   __shared__ double red[132];
   const int tid = threadIdx.x, c = tid % C;
   // part 1: rows no kernel of a solve writes (coil maps, deapodization); part 2: the rest
-  auto issue = [&](int i0, int part) {
-    const size_t off = static_cast<size_t>(i0) * N;
+  const int i0 = blockIdx.x;
+  const size_t off = static_cast<size_t>(i0) * N;
+  auto issue = [&](int part) {
     if (epi_smem && (part & 1)) {
       if (f.smaps)
         for (int cc = 0; cc < C; ++cc)
@@ -970,111 +957,105 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
     }
     cp_async_commit();
   };
-  if (blockIdx.x < lines) issue(blockIdx.x, 1);
+  issue(1);
   pdl_wait();
-  if (blockIdx.x < lines) issue(blockIdx.x, 2);
+  issue(2);
   float factor;
   if (mode == 2) factor = f.gs() / st->sigma[iter] * inv_scale2;
   else if (mode == 3 || mode == 5) factor = f.gs() / st->sigma_x * inv_scale2;
   else factor = inv_scale2 / st->sigma_y;
-  for (int i0 = blockIdx.x; i0 < lines; i0 += gridDim.x) {
-    if (i0 != blockIdx.x) {
-      __syncthreads();
-      issue(i0, 3);
-    }
-    const float2* src = w1 + static_cast<size_t>(i0) * C + c;
-    F::first(buf, f.tw, tid, [&](int n) {
-      return in_gap(n, f.axis_gap) ? make_float2(0.f, 0.f) : src[static_cast<size_t>(n) * lines * C];
-    });
+  const float2* src = w1 + static_cast<size_t>(i0) * C + c;
+  F::first(buf, f.tw, tid, [&](int n) {
+    return in_gap(n, f.axis_gap) ? make_float2(0.f, 0.f) : src[static_cast<size_t>(n) * lines * C];
+  });
+  __syncthreads();
+  if constexpr (F::R3 > 1) {
+    F::middle(buf, f.tw, tid);
     __syncthreads();
-    if constexpr (F::R3 > 1) {
-      F::middle(buf, f.tw, tid);
-      __syncthreads();
+  }
+  float2* img_s = buf;
+  if constexpr (rows_in_place<F>()) {
+    F::last_in_place(buf, tid);
+    cp_async_wait<0>();
+  } else {
+    float2 v[F::ITL][F::RL];
+    F::last(buf, tid, [&](int i, int j, int, float2 val) { v[i][j] = val; });
+    cp_async_wait<0>();
+    __syncthreads();  // the FFT rows are read: the region becomes the coil images [N][C+1]
+#pragma unroll
+    for (int i = 0; i < F::ITL; ++i) {
+      const int b = F::last_base(tid, i);
+      if (b < 0) continue;
+#pragma unroll
+      for (int j = 0; j < F::RL; ++j) {
+        int i1 = b + F::NL * j + f.shift;
+        if (i1 >= G) i1 -= G;
+        if (i1 < N) img_s[i1 * (C + 1) + c] = v[i][j];
+      }
     }
-    float2* img_s = buf;
-    if constexpr (rows_in_place<F>()) {
-      F::last_in_place(buf, tid);
-      cp_async_wait<0>();
+  }
+  __syncthreads();
+  double dot = 0.0, dot_r = 0.0, dot_a = 0.0, dot_rr = 0.0;
+  for (int i1 = tid; i1 < N; i1 += blockDim.x) {
+    const size_t pix = static_cast<size_t>(i0) * N + i1;
+    const float d = (epi_smem ? escale[i1] : f.scaling[pix]) * factor;
+    const int k = i1 >= f.shift ? i1 - f.shift : i1 - f.shift + G;  // the pixel's grid position
+    const float2* img = img_s + (rows_in_place<F>() ? F::out_row(k) * C : i1 * (C + 1));
+    if (!f.smaps) {  // coil images out [C][N][N]
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) out[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
+      continue;
+    }
+    if (mode == 5 && x) {  // the coil images before the combine, [C][N][N]
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) x[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
+    }
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int cc = 0; cc < C; ++cc) {
+      const float2 s = epi_smem ? emaps[cc * N + i1] : f.smaps[static_cast<size_t>(cc) * pix_n + pix];
+      acc = cadd(acc, cmulc(img[cc], s));
+    }
+    acc = cscale(acc, d);
+    if (mode == 0) {
+      out[pix] = acc;
+    } else if (mode == 1) {
+      r[pix] = acc;
+      x[pix] = make_float2(0.f, 0.f);
+      dot += static_cast<double>(acc.x) * acc.x + static_cast<double>(acc.y) * acc.y;
     } else {
-      float2 v[F::ITL][F::RL];
-      F::last(buf, tid, [&](int i, int j, int, float2 val) { v[i][j] = val; });
-      cp_async_wait<0>();
-      __syncthreads();  // the FFT rows are read: the region becomes the coil images [N][C+1]
-#pragma unroll
-      for (int i = 0; i < F::ITL; ++i) {
-        const int b = F::last_base(tid, i);
-        if (b < 0) continue;
-#pragma unroll
-        for (int j = 0; j < F::RL; ++j) {
-          int i1 = b + F::NL * j + f.shift;
-          if (i1 >= G) i1 -= G;
-          if (i1 < N) img_s[i1 * (C + 1) + c] = v[i][j];
-        }
-      }
-    }
-    __syncthreads();
-    double dot = 0.0, dot_r = 0.0, dot_a = 0.0, dot_rr = 0.0;
-    for (int i1 = tid; i1 < N; i1 += blockDim.x) {
-      const size_t pix = static_cast<size_t>(i0) * N + i1;
-      const float d = (epi_smem ? escale[i1] : f.scaling[pix]) * factor;
-      const int k = i1 >= f.shift ? i1 - f.shift : i1 - f.shift + G;  // the pixel's grid position
-      const float2* img = img_s + (rows_in_place<F>() ? F::out_row(k) * C : i1 * (C + 1));
-      if (!f.smaps) {  // coil images out [C][N][N]
-#pragma unroll
-        for (int cc = 0; cc < C; ++cc) out[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
-        continue;
-      }
-      if (mode == 5 && x) {  // the coil images before the combine, [C][N][N]
-#pragma unroll
-        for (int cc = 0; cc < C; ++cc) x[static_cast<size_t>(cc) * pix_n + pix] = cscale(img[cc], d);
-      }
-      float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int cc = 0; cc < C; ++cc) {
-        const float2 s = epi_smem ? emaps[cc * N + i1] : f.smaps[static_cast<size_t>(cc) * pix_n + pix];
-        acc = cadd(acc, cmulc(img[cc], s));
-      }
-      acc = cscale(acc, d);
-      if (mode == 0) {
+      const float2 pv = epi_smem ? eprow[i1] : p[pix];
+      acc.x += lambda_scaled * pv.x;
+      acc.y += lambda_scaled * pv.y;
+      if (mode == 2 || mode == 5) {
         out[pix] = acc;
-      } else if (mode == 1) {
-        r[pix] = acc;
-        x[pix] = make_float2(0.f, 0.f);
-        dot += static_cast<double>(acc.x) * acc.x + static_cast<double>(acc.y) * acc.y;
-      } else {
-        const float2 pv = epi_smem ? eprow[i1] : p[pix];
-        acc.x += lambda_scaled * pv.x;
-        acc.y += lambda_scaled * pv.y;
-        if (mode == 2 || mode == 5) {
-          out[pix] = acc;
-          dot += static_cast<double>(pv.x) * acc.x + static_cast<double>(pv.y) * acc.y;
-          if (mode == 2 && r) {
-            const float2 rv = epi_smem ? errow[i1] : r[pix];
-            dot_r += static_cast<double>(rv.x) * acc.x + static_cast<double>(rv.y) * acc.y;
-            dot_a += static_cast<double>(acc.x) * acc.x + static_cast<double>(acc.y) * acc.y;
-            dot_rr += static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
-          }
-        } else {  // reliable residual r = b - M v (b read through x)
-          const float2 bv = epi_smem ? errow[i1] : x[pix];
-          const float2 rv = make_float2(bv.x - acc.x, bv.y - acc.y);
-          out[pix] = rv;
-          dot += static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
+        dot += static_cast<double>(pv.x) * acc.x + static_cast<double>(pv.y) * acc.y;
+        if (mode == 2 && r) {
+          const float2 rv = epi_smem ? errow[i1] : r[pix];
+          dot_r += static_cast<double>(rv.x) * acc.x + static_cast<double>(rv.y) * acc.y;
+          dot_a += static_cast<double>(acc.x) * acc.x + static_cast<double>(acc.y) * acc.y;
+          dot_rr += static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
         }
+      } else {  // reliable residual r = b - M v (b read through x)
+        const float2 bv = epi_smem ? errow[i1] : x[pix];
+        const float2 rv = make_float2(bv.x - acc.x, bv.y - acc.y);
+        out[pix] = rv;
+        dot += static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
       }
     }
-    if (mode == 2 && r) {
-      const double t = warp_sum4(dot, dot_r, dot_a, dot_rr);
-      if ((tid & 7) == 0) red[(tid >> 3 & 3) * 32 + (tid >> 5)] = t;
-      __syncthreads();
-      if (tid < 4) {
-        double total = 0.0;
-        for (int w = 0; w < F::THREADS / 32; ++w) total += red[tid * 32 + w];
-        parts[tid * static_cast<int64_t>(lines) + i0] = total;
-      }
-    } else if (mode != 0) {
-      const double t = block_sum(dot, red);
-      if (tid == 0) parts[i0] = t;
+  }
+  if (mode == 2 && r) {
+    const double t = warp_sum4(dot, dot_r, dot_a, dot_rr);
+    if ((tid & 7) == 0) red[(tid >> 3 & 3) * 32 + (tid >> 5)] = t;
+    __syncthreads();
+    if (tid < 4) {
+      double total = 0.0;
+      for (int w = 0; w < F::THREADS / 32; ++w) total += red[tid * 32 + w];
+      parts[tid * static_cast<int64_t>(lines) + i0] = total;
     }
+  } else if (mode != 0) {
+    const double t = block_sum(dot, red);
+    if (tid == 0) parts[i0] = t;
   }
 }
 
@@ -1175,16 +1156,6 @@ static int sm_count() {
   return n;
 }
 
-// One CTA per item; batched cases (share > 1) run on a 1/share slice of the resident CTAs and
-// loop, so that kernels of other cases run beside them.
-template <class K>
-static int fft_grid(K k, int threads, size_t smem, int items, int share) {
-  if (share <= 1) return std::max(1, items);
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
-  return std::max(1, std::min(items, std::max(1, per_sm) * sm_count() / share));
-}
-
 #define TSN_G_SWITCH(G_, ...)                                  \
   switch (G_) {                                                \
     case 128: { constexpr int GG = 128; __VA_ARGS__; } break;  \
@@ -1218,7 +1189,7 @@ void launch_fwd_rows(const FftArgs& f, const float2* x, float2* z1, int mode, fl
     constexpr int T = LineFft<GG, CC, false>::THREADS;
     auto k = fwd_rows_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, f.pdl, f, x, z1, mode, p, r, partials, nparts, st,
+    launch_k(k, f.lines(), T, sm, s, f.pdl, f, x, z1, mode, p, r, partials, nparts, st,
              iter, xs, ap, stage);
   }));
 }
@@ -1229,7 +1200,7 @@ void launch_fwd_cols(const FftArgs& f, const float2* z1, __half* panel, cudaStre
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = fwd_cols_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, f.pdl, f, z1, panel);
+    launch_k(k, f.gcols() * (CC / W), T, sm, s, f.pdl, f, z1, panel);
   }));
 }
 
@@ -1239,7 +1210,7 @@ void launch_fwd_mid(const FftArgs& f, const float2* z1, float2* z2, cudaStream_t
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = fwd_mid_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, f.pdl, f, z1, z2);
+    launch_k(k, f.N * f.G * (CC / W), T, sm, s, f.pdl, f, z1, z2);
   }));
 }
 
@@ -1249,7 +1220,7 @@ void launch_inv_mid(const FftArgs& f, const float2* z2, float2* z1, cudaStream_t
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = inv_mid_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.N * f.G * (CC / W), f.share), T, sm, s, f.pdl, f, z2, z1);
+    launch_k(k, f.N * f.G * (CC / W), T, sm, s, f.pdl, f, z2, z1);
   }));
 }
 
@@ -1266,7 +1237,7 @@ void launch_inv_cols(const FftArgs& f, const float2* grid, float2* w1, cudaStrea
     const size_t sm = fft_rows_bytes<GG, W>();
     auto k = inv_cols_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.gcols() * (CC / W), f.share), T, sm, s, f.pdl, f, grid, w1);
+    launch_k(k, f.gcols() * (CC / W), T, sm, s, f.pdl, f, grid, w1);
   }));
 }
 
@@ -1283,7 +1254,7 @@ void launch_inv_rows(const FftArgs& f, const float2* w1, float2* out, int mode, 
     constexpr int T = LineFft<GG, CC, true>::THREADS;
     auto k = inv_rows_kernel<GG, CC>;
     ensure_smem(k, sm);
-    launch_k(k, fft_grid(k, T, sm, f.lines(), f.share), T, sm, s, f.pdl, f, w1, out, mode, x, r, p, partials, st, iter,
+    launch_k(k, f.lines(), T, sm, s, f.pdl, f, w1, out, mode, x, r, p, partials, st, iter,
              inv_scale2, lambda_scaled, static_cast<int>(region), epi_smem);
   }));
 }

@@ -105,7 +105,6 @@ struct FftArgs {
   const float2* tw = nullptr;           // exp(-2 pi i e/G), e in [0,G)
   const float* scaling = nullptr;       // [N]^dims deapodization
   const float2* smaps = nullptr;        // [C][N]^dims or null
-  int share = 1;                        // persistent grids use 1/share of the resident CTAs
   int dims = 2;                         // 2: image [N][N]; 3: volume [N][N][N]
   bool pdl = false;                     // launch with programmatic dependent launch (direct calls)
   bool maps_early = true;               // forward rows may read the coil maps ahead of pdl_wait: a kernel of

@@ -634,7 +634,7 @@ bool direct_pdl(cudaStream_t s) {
 
 // gaps: leave out the grid cells that no sample touches (everything but the FFT endpoints, whose
 // callers own the whole grid)
-FftArgs fft_args(const tsn_plan* P, const void* smaps, int share = 1, bool pdl = false, bool gaps = true) {
+FftArgs fft_args(const tsn_plan* P, const void* smaps, bool pdl = false, bool gaps = true) {
   FftArgs f;
   if (gaps) {
     f.cell_gap = P->cell_gap.as<int2>();
@@ -642,7 +642,6 @@ FftArgs fft_args(const tsn_plan* P, const void* smaps, int share = 1, bool pdl =
     f.axis_gap = P->axis_gap;
   }
   f.pdl = pdl;
-  f.share = share;
   f.N = P->N;
   f.G = P->G;
   f.C = P->C;
@@ -1093,7 +1092,7 @@ void run_interp(const tsn_plan* P, int which, int share, int epi, const InterpOu
 }
 
 void enqueue_forward(tsn_plan* P, const void* x, const void* smaps, void* y, cudaStream_t s, bool reference = false) {
-  const FftArgs f = fft_args(P, smaps, 1, direct_pdl(s));
+  const FftArgs f = fft_args(P, smaps, direct_pdl(s));
   CgState* st = P->state.as<CgState>();
   const int64_t n = image_pixels(P) * (smaps ? 1 : P->C);
   launch_norm_partials(static_cast<const float2*>(x), n, P->norm_parts.as<double>(), s, f.pdl);
@@ -1117,7 +1116,7 @@ static_assert(kCgStepParts == TSN_CG_STEP_PARTS, "CG-step partial count of the k
 
 void enqueue_normal(tsn_plan* P, const void* p, const void* smaps, const float* density, float lambda, void* q,
                     void* coils, double* pq, const double* p_parts, int n_p_parts, cudaStream_t s) {
-  FftArgs f = fft_args(P, smaps, 1, direct_pdl(s));
+  FftArgs f = fft_args(P, smaps, direct_pdl(s));
   f.maps_early = p_parts == nullptr;  // else the forward rows are the call's first kernel
   CgState* st = P->state.as<CgState>();
   const float2* pv = static_cast<const float2*>(p);
@@ -1190,7 +1189,7 @@ void enqueue_cg(tsn_plan* P, const void* y, const void* smaps, const float* dens
   auto ref_step = [&](int k) {  // iteration k (0-based) completes iteration k + 1
     return have_ref && ((k < 64 && ((ref_steps >> k) & 1ull)) || (ref_period > 0 && (k + 1) % ref_period == 0));
   };
-  const FftArgs f = fft_args(P, smaps, share);
+  const FftArgs f = fft_args(P, smaps);
   CgState* st = P->state.as<CgState>();
   const float inv_s2 = 1.0f / (scale * scale);
   const float lam = lambda * inv_s2;
@@ -1313,7 +1312,7 @@ static tsn_status adjoint_entry(tsn_plan* plan, const void* y, const void* smaps
     if (reference && !plan->view_ref[TSN_VIEW_GT].present)
       fail(TSN_ERR_ARG, "the reference operator needs a plan built with TSN_FLAG_REFERENCE_STEPS");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const FftArgs f = fft_args(plan, smaps, 1, direct_pdl(s));
+    const FftArgs f = fft_args(plan, smaps, direct_pdl(s));
     enqueue_adjoint_grid(plan, y, nullptr, s, 1, reference, f.pdl);
     inv_to_lines(plan, f, plan->grid.as<float2>(), s);
     launch_inv_rows(f, plan->z1.as<float2>(), static_cast<float2*>(x), 0, nullptr, nullptr, nullptr, nullptr,
@@ -1724,7 +1723,7 @@ tsn_status tsn_fft_forward_panel(tsn_plan* plan, const void* x, const void* smap
     need_aligned({x, smaps, panel_f16});
     need_views(plan, false, false);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const FftArgs f = fft_args(plan, smaps, 1, false, false);
+    const FftArgs f = fft_args(plan, smaps, false, false);
     CgState* st = plan->state.as<CgState>();
     const int64_t n = image_pixels(plan) * (smaps ? 1 : plan->C);
     launch_norm_partials(static_cast<const float2*>(x), n, plan->norm_parts.as<double>(), s);
@@ -1750,7 +1749,7 @@ tsn_status tsn_fft_adjoint_image(tsn_plan* plan, const void* grid_c64, const voi
     need_aligned({grid_c64, smaps, x});
     need_views(plan, false, false);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const FftArgs f = fft_args(plan, smaps, 1, false, false);
+    const FftArgs f = fft_args(plan, smaps, false, false);
     CgState* st = plan->state.as<CgState>();
     // unit sample scale for the plain adjoint epilogue (factor = 1 / sigma_y)
     const float one = 1.0f;
