@@ -261,6 +261,36 @@ tsn_status tsn_cg_adjoint_step(tsn_plan* plan, int64_t n, const double* rho, con
 tsn_status tsn_cg_adjoint_finish(tsn_plan* plan, int64_t n, int32_t coils, void* pb, const void* mqb,
                                  const void* qb, const void* coil_images, const void* coil_images_bar,
                                  const void* p, void* sb, tsn_stream_t stream);
+/* The steps of a differentiable unrolled solve, enqueued by one call each (the loops of
+ * tsn_normal with tsn_cg_step, and of tsn_normal with tsn_cg_adjoint_step and _finish, without a
+ * host call per step).  iters >= 1, checkpoint >= 1, segments = ceil(iters / checkpoint).
+ * Images hold n complex64 (one plan image), device pointers 16-byte aligned.
+ *
+ * tsn_cg_unrolled runs `iters` iterations of M = A^H W A + lambda from x, r, p in states[0]:
+ *   states       [segments][3][n]  x, r, p before iterations 0, checkpoint, 2 checkpoint, ...
+ *                                  (states[0] is given, the others are written)
+ *   rho, gamma   [iters + 1], [iters] device doubles: |r_k|^2 (rho[0] given), Re <p_k, M p_k>
+ *   q            [segments][n]     M p of each segment's first iteration
+ *   coil_images  [segments][C][n]  its coil images A_c^H W A p, or NULL
+ *   work         TSN_CG_UNROLLED_WORK(n) bytes
+ *   x            [n]               the last iterate
+ * tsn_cg_unrolled_adjoint runs the reverse steps over the same arrays, recomputing each
+ * segment from its checkpoint: xb (cotangent of x) is read; rb, pb (cotangents of r and p, zero
+ * or the last step's) are updated in place to those of states[0]; rhob[0] is the cotangent of
+ * rho[iters], rhob[iters & 1] ends as that of rho[0]; with sb != NULL (needs coil_images) the
+ * coil-map cotangent [C][n] is added to it.  work: TSN_CG_UNROLLED_ADJOINT_WORK bytes. */
+#define TSN_CG_UNROLLED_WORK(n) (7 * 8 * (int64_t)(n) + 8 * TSN_CG_STEP_PARTS)
+#define TSN_CG_UNROLLED_ADJOINT_WORK(n, coils, checkpoint, with_maps)                                       \
+  (8 * (int64_t)(n) * (3 * (int64_t)(checkpoint) + 3 + ((with_maps) ? ((int64_t)(checkpoint) + 1) * (coils) : 0)) + \
+   8 * (2 * TSN_CG_STEP_PARTS + 2))
+tsn_status tsn_cg_unrolled(tsn_plan* plan, const void* smaps, const float* density, float lambda,
+                           int32_t iters, int32_t checkpoint, void* states, double* rho, double* gamma,
+                           void* q, void* coil_images, void* work, void* x, tsn_stream_t stream);
+tsn_status tsn_cg_unrolled_adjoint(tsn_plan* plan, const void* smaps, const float* density, float lambda,
+                                   int32_t iters, int32_t checkpoint, const void* states, const double* rho,
+                                   const double* gamma, const void* q, const void* coil_images,
+                                   const void* xb, void* rb, void* pb, void* sb, double* rhob, void* work,
+                                   tsn_stream_t stream);
 /* The FP32-class operators of a plan built with TSN_FLAG_REFERENCE_STEPS (the reference's
  * forward_reference / adjoint_reference, reference_sparse_solver.py:590-630, which its CG uses
  * for scheduled reference steps): same arguments and units as tsn_forward / tsn_adjoint, every

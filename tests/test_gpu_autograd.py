@@ -250,3 +250,41 @@ def test_fused_backward_matches_composed_backward():
         grads.append([t.grad.cpu().numpy() for t in leaves])
     for a, b in zip(*grads):
         assert np.linalg.norm(a - b) <= 1e-3 * np.linalg.norm(b)
+
+
+class _StepOps:
+    """A plan's operator pieces with one host call per CG step (no native loop)."""
+
+    def __init__(self, plan):
+        from trajsparsenufft_b200 import autograd as tad
+        ops = tad.PlanOps(plan)
+        for name in ("forward_coils", "adjoint_coils", "normal", "rdot", "forward_maps", "step", "adjoint_step",
+                     "adjoint_finish"):
+            setattr(self, name, getattr(ops, name))
+
+
+# one segment, segments of one step, a short last segment, whole segments; with and without map
+# gradients, density and a nonzero start
+@pytest.mark.parametrize("iters,checkpoint,need_s,density,start", [
+    (1, 1, True, False, False), (3, 1, True, True, False), (5, 2, True, False, True), (4, 2, False, False, False),
+    (6, 4, True, False, False), (3, 8, True, True, True)])
+def test_native_unrolled_solve_matches_stepwise(iters, checkpoint, need_s, density, start):
+    """The native loops run the step-wise path's kernels on the same values (a segment's last
+    residual is read from the next checkpoint instead of being recomputed, the curvature is the
+    forward's): images and gradients agree to FP32 rounding grown by the solve."""
+    from gpu_cases import torch_inputs
+    from trajsparsenufft_b200 import autograd as tad, synth
+    from trajsparsenufft_b200.operator import Plan
+    traj, x, s, n, g, c, j, readout = case("small")
+    plan = Plan.from_trajectory(traj, im_size=n, grid_size=g, coils=c, width=j)
+    xt, st, yt = torch_inputs("small")
+    w = torch.from_numpy(synth.ramp_density(traj, readout)).cuda() if density else None
+    got = []
+    for ops in (tad.PlanOps(plan), _StepOps(plan)):
+        y, sm = yt.clone().requires_grad_(True), st.clone().requires_grad_(need_s)
+        x0 = (0.3 * xt if start else torch.zeros_like(xt)).requires_grad_(True)
+        xk = tad.cg_sense(y, sm, ops, x0=x0, density=w, lam=1e-4, iters=iters, checkpoint=checkpoint)
+        (xk - xt).abs().pow(2).sum().backward()
+        got.append([v.detach() for v in (xk, y.grad, x0.grad) + ((sm.grad,) if need_s else ())])
+    for a, b in zip(*got):
+        assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b)) <= 1e-4

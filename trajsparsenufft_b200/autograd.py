@@ -68,6 +68,15 @@ class PlanOps:
         |qb|^2 partials)."""
         return self.plan.cg_adjoint_step(rho, rho_n, gamma, rhob, rb, pb, p, q, r_n, xb, norm_parts=True)
 
+    def unrolled(self, x0, r0, rho0, smaps, density, lam, iters, checkpoint, coils):
+        """All CG steps in one call: (x, tensors for unrolled_adjoint)."""
+        return self.plan.cg_unrolled(x0.contiguous(), r0.contiguous(), rho0, smaps.contiguous(), density, lam, iters,
+                                     checkpoint, coils)
+
+    def unrolled_adjoint(self, saved, smaps, density, lam, iters, checkpoint, xb, sb):
+        """All reverse steps in one call: (rb, pb, rhob) at the start, sb in place."""
+        return self.plan.cg_unrolled_adjoint(saved, smaps.contiguous(), density, lam, iters, checkpoint, xb, sb)
+
     def adjoint_finish(self, pb, mqb, qb=None, t=None, tb=None, p=None, sb=None):
         """pb += M qb and the coil-map cotangent update, in place."""
         self.plan.cg_adjoint_finish(pb, mqb, qb, t, tb, p, sb)
@@ -203,6 +212,14 @@ class UnrolledCgSense(torch.autograd.Function):
         b = S.combine(u)
         if x0_zero is None:                        # decided from the values (a host sync)
             x0_zero = not bool(x0.abs().amax() > 0)
+        if S.fused and iters > 0 and hasattr(ops, "unrolled"):  # every step in one native call
+            r = b if x0_zero else b - S.M(x0)
+            x, saved = ops.unrolled(x0, r, S.dot(r, r), smaps, density, lam, iters, checkpoint, ctx.needs_input_grad[1])
+            ctx.ops, ctx.lam, ctx.iters, ctx.checkpoint, ctx.x0_zero = ops, lam, iters, checkpoint, x0_zero
+            ctx.has_density, ctx.native = density is not None, True
+            ctx.save_for_backward(smaps, x0, u, *(() if density is None else (density,)), *saved)
+            return x
+        ctx.native = False
         x = x0.clone()
         r = b.clone() if x0_zero else b - S.M(x0)
         p = r.clone()
@@ -235,13 +252,19 @@ class UnrolledCgSense(torch.autograd.Function):
         smaps, x0, u = saved[0], saved[1], saved[2]
         density = saved[3] if ctx.has_density else None
         flat = saved[4 if ctx.has_density else 3:]
+        if ctx.native:
+            S = _Sense(ctx.ops, smaps, density, ctx.lam)
+            xb = gx.contiguous()
+            sb = torch.zeros_like(smaps, memory_format=torch.contiguous_format) if ctx.needs_input_grad[1] else None
+            rb, pb, rhob = ctx.ops.unrolled_adjoint(flat, smaps, density, ctx.lam, ctx.iters, ctx.checkpoint, xb, sb)
+            return UnrolledCgSense._start_gradients(ctx, S, smaps, x0, u, xb, rb, pb, rhob, flat[0][0, 1], sb)
         n_seg = (ctx.iters + ctx.checkpoint - 1) // ctx.checkpoint   # segments (firsts)
         n_cp = max(1, n_seg)                                          # checkpoints incl. the start
         cps = [tuple(flat[i:i + 4]) for i in range(0, 4 * n_cp, 4)]
         fw = ctx.first_width
         firsts = [tuple(flat[4 * n_cp + i:4 * n_cp + i + fw]) for i in range(0, fw * n_seg, fw)]
         S = _Sense(ctx.ops, smaps, density, ctx.lam)
-        need_y, need_s, need_x0 = ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_input_grad[2]
+        need_s = ctx.needs_input_grad[1]
         c, iters = ctx.checkpoint, ctx.iters
         xb = gx.contiguous()
         rb = torch.zeros_like(xb)
@@ -296,8 +319,13 @@ class UnrolledCgSense(torch.autograd.Function):
                     mqb = S.M(qb)
                 pb = pbk + mqb
                 rhob = rhobk
+        return UnrolledCgSense._start_gradients(ctx, S, smaps, x0, u, xb, rb, pb, rhob, cps[0][1], sb)
+
+    @staticmethod
+    def _start_gradients(ctx, S, smaps, x0, u, xb, rb, pb, rhob, r0, sb):
+        """From the cotangents at the start of the solve to those of y, the maps and x0."""
+        need_y, need_s, need_x0 = ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_input_grad[2]
         # p0 = r0, rho0 = |r0|^2, r0 = b - M x0
-        r0 = cps[0][1]
         rb = rb + pb + (2.0 * rhob) * r0
         gy = gs = gx0 = None
         if need_x0:

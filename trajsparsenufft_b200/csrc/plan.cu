@@ -1424,6 +1424,98 @@ tsn_status tsn_cg_adjoint_finish(tsn_plan* plan, int64_t n, int32_t coils, void*
   }
 }
 
+tsn_status tsn_cg_unrolled(tsn_plan* plan, const void* smaps, const float* density, float lambda, int32_t iters,
+                           int32_t checkpoint, void* states, double* rho, double* gamma, void* q, void* coil_images,
+                           void* work, void* x, tsn_stream_t stream) {
+  try {
+    if (!plan || !smaps || !states || !rho || !gamma || !q || !work || !x) fail(TSN_ERR_ARG, "NULL argument");
+    if (iters < 1 || checkpoint < 1) fail(TSN_ERR_ARG, "iters and checkpoint must be >= 1");
+    if (!std::isfinite(lambda)) fail(TSN_ERR_ARG, "lambda must be finite");
+    need_aligned({smaps, density, states, q, coil_images, work, x});
+    need_views(plan, true, true);
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const int64_t n = image_pixels(plan);
+    float2 *st = static_cast<float2*>(states), *w = static_cast<float2*>(work), *qs = static_cast<float2*>(q);
+    float2 *ts = static_cast<float2*>(coil_images), *q_tmp = w + 6 * n;
+    double* parts = reinterpret_cast<double*>(w + 7 * n);
+    const float2* cur = st;  // x, r, p of iteration k
+    for (int32_t k = 0; k < iters; ++k) {
+      const int64_t seg = k / checkpoint;
+      const bool first = k % checkpoint == 0, last = k + 1 == iters;
+      float2* qk = first ? qs + seg * n : q_tmp;
+      enqueue_normal(plan, cur + 2 * n, smaps, density, lambda, qk, first && ts ? ts + seg * plan->C * n : nullptr,
+                     gamma + k, k > 0 ? parts : nullptr, kCgStepParts, s);
+      float2* next = !last && (k + 1) % checkpoint == 0 ? st + (seg + 1) * 3 * n : w + (k & 1) * 3 * n;
+      launch_cg_step(n, plan->adj_parts.as<double>(), rho + k, gamma + k, cur, cur + 2 * n, cur + n, qk,
+                     last ? static_cast<float2*>(x) : next, next + n, next + 2 * n, rho + k + 1, parts, s, direct_pdl(s));
+      cur = next;
+    }
+    CUDA_OK(cudaGetLastError());
+    return TSN_OK;
+  } catch (const std::exception& e) {
+    return guard_status(e);
+  }
+}
+
+tsn_status tsn_cg_unrolled_adjoint(tsn_plan* plan, const void* smaps, const float* density, float lambda, int32_t iters,
+                                   int32_t checkpoint, const void* states, const double* rho, const double* gamma,
+                                   const void* q, const void* coil_images, const void* xb, void* rb, void* pb, void* sb,
+                                   double* rhob, void* work, tsn_stream_t stream) {
+  try {
+    if (!plan || !smaps || !states || !rho || !gamma || !q || !xb || !rb || !pb || !rhob || !work)
+      fail(TSN_ERR_ARG, "NULL argument");
+    if (sb && !coil_images) fail(TSN_ERR_ARG, "the map cotangent needs the coil images");
+    if (iters < 1 || checkpoint < 1) fail(TSN_ERR_ARG, "iters and checkpoint must be >= 1");
+    if (!std::isfinite(lambda)) fail(TSN_ERR_ARG, "lambda must be finite");
+    need_aligned({smaps, density, states, q, coil_images, xb, rb, pb, sb, work});
+    need_views(plan, true, true);
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const bool pdl = direct_pdl(s);
+    const int64_t n = image_pixels(plan), cn = plan->C * n, cp = checkpoint;
+    const float2 *st = static_cast<const float2*>(states), *qs = static_cast<const float2*>(q);
+    const float2* ts = static_cast<const float2*>(coil_images);
+    // work: p [cp + 1], r' [cp], q [cp], then q-bar, M q-bar, and with maps t [cp][C], t-bar [C]
+    float2* wp = static_cast<float2*>(work);
+    float2 *wr = wp + (cp + 1) * n, *wq = wr + cp * n, *qb = wq + cp * n, *mqb = qb + n, *wt = mqb + n;
+    float2* tb = wt + (sb ? cp * cn : 0);
+    double* parts = reinterpret_cast<double*>(tb + (sb ? cn : 0));
+    double *qb_parts = parts + kCgStepParts, *rho_tmp = qb_parts + kCgStepParts, *tmp = plan->adj_parts.as<double>();
+    int cur = 0;
+    for (int64_t seg = (iters - 1) / cp; seg >= 0; --seg) {
+      const int64_t k0 = seg * cp, k1 = std::min<int64_t>(k0 + cp, iters);
+      auto p_at = [&](int64_t j) { return j == 0 ? st + (3 * seg + 2) * n : wp + j * n; };
+      auto q_at = [&](int64_t j) { return j == 0 ? qs + seg * n : wq + j * n; };
+      auto t_at = [&](int64_t j) { return j == 0 ? ts + seg * cn : wt + j * cn; };
+      // r' of the segment's last step is the next checkpoint's r
+      auto r_at = [&](int64_t j) { return k0 + j + 1 == k1 && k1 < iters ? st + (3 * (seg + 1) + 1) * n : wr + j * n; };
+      const float2* r = st + (3 * seg + 1) * n;
+      for (int64_t k = k0; k < k1; ++k) {  // the segment's states again
+        const int64_t j = k - k0;
+        if (j > 0)
+          enqueue_normal(plan, p_at(j), smaps, density, lambda, wq + j * n, sb ? wt + j * cn : nullptr, nullptr, parts,
+                         kCgStepParts, s);
+        if (k + 1 < k1 || k1 == iters)
+          launch_cg_step(n, tmp, rho + k, gamma + k, nullptr, p_at(j), r, q_at(j), nullptr, wr + j * n, wp + (j + 1) * n,
+                         rho_tmp, parts, s, pdl);
+        r = r_at(j);
+      }
+      for (int64_t k = k1 - 1; k >= k0; --k, cur ^= 1) {
+        const int64_t j = k - k0;
+        launch_cg_adjoint_step(n, tmp, rho + k, rho + k + 1, gamma + k, rhob + cur, rhob + (cur ^ 1),
+                               static_cast<float2*>(rb), static_cast<float2*>(pb), p_at(j), q_at(j), r_at(j),
+                               static_cast<const float2*>(xb), qb, qb_parts, s, pdl);
+        enqueue_normal(plan, qb, smaps, density, lambda, mqb, sb ? tb : nullptr, nullptr, qb_parts, kCgStepParts, s);
+        launch_cg_adjoint_finish(n, sb ? plan->C : 0, static_cast<float2*>(pb), mqb, qb, sb ? t_at(j) : nullptr, tb,
+                                 p_at(j), static_cast<float2*>(sb), s, pdl);
+      }
+    }
+    CUDA_OK(cudaGetLastError());
+    return TSN_OK;
+  } catch (const std::exception& e) {
+    return guard_status(e);
+  }
+}
+
 tsn_status tsn_forward_reference(tsn_plan* plan, const void* x, const void* smaps, void* y, tsn_stream_t stream) {
   return forward_entry(plan, x, smaps, y, stream, true);
 }

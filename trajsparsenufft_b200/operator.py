@@ -285,6 +285,53 @@ class Plan:
                      _dev_ptr(p, cf, shape, "p"), _dev_ptr(sb, cf, cshape, "sb")]
         check(lib().tsn_cg_adjoint_finish(self._h, int(pb.numel()), int(coils), *args, _stream_handle(stream)))
 
+    def cg_unrolled(self, x0, r0, rho0, smaps, density, lam, iters, checkpoint, coils, stream=None):
+        """`iters` CG steps of A^H W A + lam from x0 with p0 = r0 and rho0 = |r0|^2 (0-d FP64), in
+        one call (tsn_cg_unrolled).  Returns (x, the saved tensors that cg_unrolled_adjoint
+        takes); coils=True saves the coil images that the map cotangent needs."""
+        torch = _torch()
+        cf, dev, shape = torch.complex64, r0.device, self.image_shape
+        for t, name in ((x0, "x0"), (r0, "r0")):
+            _dev_ptr(t, cf, shape, name)
+        sp = _dev_ptr(smaps, cf, self.maps_shape, "smaps")
+        dp = None if density is None else _dev_ptr(density, torch.float32, (self.samples,), "density")
+        seg, n = -(-iters // checkpoint), r0.numel()
+        states = torch.empty((seg, 3) + shape, dtype=cf, device=dev)
+        states[0, 0] = x0
+        states[0, 1:] = r0
+        rho, gamma = (torch.empty(k, dtype=torch.float64, device=dev) for k in (iters + 1, iters))
+        rho[0] = rho0
+        q = torch.empty((seg,) + shape, dtype=cf, device=dev)
+        t = torch.empty((seg,) + self.maps_shape, dtype=cf, device=dev) if coils else None
+        work = torch.empty(7 * 8 * n + 8 * _lib.CG_STEP_PARTS, dtype=torch.uint8, device=dev)
+        x = torch.empty(shape, dtype=cf, device=dev)
+        at = lambda v: None if v is None else C.c_void_p(v.data_ptr())
+        check(lib().tsn_cg_unrolled(self._h, sp, dp, float(lam), int(iters), int(checkpoint), at(states), at(rho), at(gamma),
+                                    at(q), at(t), at(work), at(x), _stream_handle(stream)))
+        return x, (states, rho, gamma, q) + (() if t is None else (t,))
+
+    def cg_unrolled_adjoint(self, saved, smaps, density, lam, iters, checkpoint, xb, sb=None, stream=None):
+        """The reverse steps of cg_unrolled (tsn_cg_unrolled_adjoint): returns the cotangents of r0
+        (rb), p0 (pb) and rho0 (a 0-d FP64 device tensor); with sb given, the coil-map cotangent
+        is added to it in place."""
+        torch = _torch()
+        cf, dev, shape = torch.complex64, xb.device, self.image_shape
+        states, rho, gamma, q = saved[:4]
+        sp = _dev_ptr(smaps, cf, self.maps_shape, "smaps")
+        dp = None if density is None else _dev_ptr(density, torch.float32, (self.samples,), "density")
+        xp = _dev_ptr(xb, cf, shape, "xb")
+        bp = None if sb is None else _dev_ptr(sb, cf, self.maps_shape, "sb")
+        n = xb.numel()
+        images = 3 * checkpoint + 3 + ((checkpoint + 1) * self.coils if sb is not None else 0)
+        work = torch.empty(8 * n * images + 8 * (2 * _lib.CG_STEP_PARTS + 2), dtype=torch.uint8, device=dev)
+        rb, pb = torch.zeros_like(xb), torch.zeros_like(xb)
+        rhob = torch.zeros(2, dtype=torch.float64, device=dev)
+        at = lambda v: C.c_void_p(v.data_ptr())
+        check(lib().tsn_cg_unrolled_adjoint(self._h, sp, dp, float(lam), int(iters), int(checkpoint), at(states), at(rho),
+                                            at(gamma), at(q), at(saved[4]) if sb is not None else None, xp, at(rb), at(pb),
+                                            bp, at(rhob), at(work), _stream_handle(stream)))
+        return rb, pb, rhob[iters & 1]
+
     def cg_sense(self, y, smaps, *, density=None, lam=1e-4, iters=10, operator_scale=1.0, out=None, stream=None,
                  sync=True, reliable_update_period=0, reliable_update_direction="restart",
                  scheduled_reference_period=0, reference_steps=()):
