@@ -288,3 +288,33 @@ def test_native_unrolled_solve_matches_stepwise(iters, checkpoint, need_s, densi
         got.append([v.detach() for v in (xk, y.grad, x0.grad) + ((sm.grad,) if need_s else ())])
     for a, b in zip(*got):
         assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b)) <= 1e-4
+
+
+def test_native_unrolled_solve_on_another_stream():
+    """With stream= the loops run on that stream behind the current one, which is kept busy here, so
+    arrays filled on it would be read too early; allocations on the current stream right after the
+    calls must not get the memory of arrays still in use.  The same kernels on the same values:
+    equal bits."""
+    from gpu_cases import torch_inputs
+    from trajsparsenufft_b200.operator import Plan
+    traj, x, s, n, g, c, j, _ = case("small")
+    plan = Plan.from_trajectory(traj, im_size=n, grid_size=g, coils=c, width=j)
+    xt, st, yt = torch_inputs("small")
+    x0, r0 = 0.3 * xt, plan.adjoint(yt, st)
+    rho0 = plan.rdot(r0, r0)
+    torch.cuda.synchronize()
+    side, got = torch.cuda.Stream(), []
+    for stream in (None, side):
+        sb = torch.zeros_like(st)
+        torch.cuda._sleep(20_000_000)  # about 10 ms of the current stream
+        xk, saved = plan.cg_unrolled(x0, r0, rho0, st, None, LAM, 5, 2, True, stream=stream)
+        junk = [torch.full((1 << 18,), float("nan"), device="cuda") for _ in range(8)]
+        if stream is not None:
+            stream.wait_stream(torch.cuda.current_stream())
+        torch.cuda._sleep(20_000_000)
+        back = plan.cg_unrolled_adjoint(saved, st, None, LAM, 5, 2, (xk if stream is None else got[0][0]), sb, stream=stream)
+        junk += [torch.full((1 << 18,), float("nan"), device="cuda") for _ in range(8)]
+        torch.cuda.synchronize()
+        got.append((xk, *back, sb))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

@@ -10,6 +10,7 @@ CPU or torch fallback.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from pathlib import Path
 
@@ -43,6 +44,25 @@ def _dev_ptr(t, dtype, shape, name):
     if t.is_complex() and t.is_conj():
         raise ValueError(f"{name} is a lazily conjugated view: pass {name}.resolve_conj()")
     return C.c_void_p(t.data_ptr())
+
+
+def _record(stream, *values):
+    """Keeps the memory of the CUDA tensors among `values` from being handed out again before the
+    work queued on `stream` when they are freed has run."""
+    for t in values:
+        if isinstance(t, _torch().Tensor) and t.is_cuda:
+            t.record_stream(stream)
+
+
+@contextlib.contextmanager
+def _run_on(stream, *inputs):
+    """torch work on `stream` behind the current stream, with the inputs kept for it: for calls that
+    fill or copy arrays of their own for a kernel on `stream`."""
+    torch = _torch()
+    stream.wait_stream(torch.cuda.current_stream())
+    _record(stream, *inputs)
+    with torch.cuda.stream(stream):
+        yield
 
 
 INTERP = {"auto": 0, "mma_sp": 1, "tcgen05": 2}
@@ -288,8 +308,14 @@ class Plan:
     def cg_unrolled(self, x0, r0, rho0, smaps, density, lam, iters, checkpoint, coils, stream=None):
         """`iters` CG steps of A^H W A + lam from x0 with p0 = r0 and rho0 = |r0|^2 (0-d FP64), in
         one call (tsn_cg_unrolled).  Returns (x, the saved tensors that cg_unrolled_adjoint
-        takes); coils=True saves the coil images that the map cotangent needs."""
+        takes); coils=True saves the coil images that the map cotangent needs.  With `stream`,
+        everything runs there, behind the current stream."""
         torch = _torch()
+        if stream is not None and stream != (cur := torch.cuda.current_stream()):
+            with _run_on(stream, x0, r0, rho0, smaps, density):
+                x, saved = self.cg_unrolled(x0, r0, rho0, smaps, density, lam, iters, checkpoint, coils)
+            _record(cur, x, *saved)
+            return x, saved
         cf, dev, shape = torch.complex64, r0.device, self.image_shape
         for t, name in ((x0, "x0"), (r0, "r0")):
             _dev_ptr(t, cf, shape, name)
@@ -307,14 +333,19 @@ class Plan:
         x = torch.empty(shape, dtype=cf, device=dev)
         at = lambda v: None if v is None else C.c_void_p(v.data_ptr())
         check(lib().tsn_cg_unrolled(self._h, sp, dp, float(lam), int(iters), int(checkpoint), at(states), at(rho), at(gamma),
-                                    at(q), at(t), at(work), at(x), _stream_handle(stream)))
+                                    at(q), at(t), at(work), at(x), _stream_handle()))
         return x, (states, rho, gamma, q) + (() if t is None else (t,))
 
     def cg_unrolled_adjoint(self, saved, smaps, density, lam, iters, checkpoint, xb, sb=None, stream=None):
         """The reverse steps of cg_unrolled (tsn_cg_unrolled_adjoint): returns the cotangents of r0
         (rb), p0 (pb) and rho0 (a 0-d FP64 device tensor); with sb given, the coil-map cotangent
-        is added to it in place."""
+        is added to it in place.  With `stream`, everything runs there, behind the current stream."""
         torch = _torch()
+        if stream is not None and stream != (cur := torch.cuda.current_stream()):
+            with _run_on(stream, *saved, smaps, density, xb, sb):
+                out = self.cg_unrolled_adjoint(saved, smaps, density, lam, iters, checkpoint, xb, sb)
+            _record(cur, *out)
+            return out
         cf, dev, shape = torch.complex64, xb.device, self.image_shape
         states, rho, gamma, q = saved[:4]
         sp = _dev_ptr(smaps, cf, self.maps_shape, "smaps")
@@ -329,7 +360,7 @@ class Plan:
         at = lambda v: C.c_void_p(v.data_ptr())
         check(lib().tsn_cg_unrolled_adjoint(self._h, sp, dp, float(lam), int(iters), int(checkpoint), at(states), at(rho),
                                             at(gamma), at(q), at(saved[4]) if sb is not None else None, xp, at(rb), at(pb),
-                                            bp, at(rhob), at(work), _stream_handle(stream)))
+                                            bp, at(rhob), at(work), _stream_handle()))
         return rb, pb, rhob[iters & 1]
 
     def cg_sense(self, y, smaps, *, density=None, lam=1e-4, iters=10, operator_scale=1.0, out=None, stream=None,
