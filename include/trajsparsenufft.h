@@ -278,7 +278,8 @@ tsn_status tsn_cg_adjoint_finish(tsn_plan* plan, int64_t n, int32_t coils, void*
  * segment from its checkpoint: xb (cotangent of x) is read; rb, pb (cotangents of r and p, zero
  * or the last step's) are updated in place to those of states[0]; rhob[0] is the cotangent of
  * rho[iters], rhob[iters & 1] ends as that of rho[0]; with sb != NULL (needs coil_images) the
- * coil-map cotangent [C][n] is added to it.  work: TSN_CG_UNROLLED_ADJOINT_WORK bytes. */
+ * coil-map cotangent [C][n] is added to it.  work: TSN_CG_UNROLLED_ADJOINT_WORK bytes, with
+ * min(checkpoint, iters) for checkpoint (a segment is at most the whole solve). */
 #define TSN_CG_UNROLLED_WORK(n) (7 * 8 * (int64_t)(n) + 8 * TSN_CG_STEP_PARTS)
 #define TSN_CG_UNROLLED_ADJOINT_WORK(n, coils, checkpoint, with_maps)                                       \
   (8 * (int64_t)(n) * (3 * (int64_t)(checkpoint) + 3 + ((with_maps) ? ((int64_t)(checkpoint) + 1) * (coils) : 0)) + \

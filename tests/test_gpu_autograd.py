@@ -318,3 +318,25 @@ def test_native_unrolled_solve_on_another_stream():
         got.append((xk, *back, sb))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_interval_beyond_the_solve_costs_no_memory():
+    """One segment, asked for by the solve's length and by fifty times it: the same peak of device
+    memory and the same bits."""
+    from gpu_cases import torch_inputs
+    from trajsparsenufft_b200 import autograd as tad
+    from trajsparsenufft_b200.operator import Plan
+    traj, x, s, n, g, c, j, _ = case("small")
+    plan = Plan.from_trajectory(traj, im_size=n, grid_size=g, coils=c, width=j)
+    _, st, yt = torch_inputs("small")
+    peaks, grads = [], []
+    for checkpoint in (4, 4, 200):  # the first warms up
+        sm = st.clone().requires_grad_(True)
+        torch.cuda.synchronize()
+        base = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        tad.cg_sense(yt, sm, tad.PlanOps(plan), lam=LAM, iters=4, checkpoint=checkpoint).abs().pow(2).sum().backward()
+        peaks.append(torch.cuda.max_memory_allocated() - base)
+        grads.append(sm.grad)
+    assert peaks[2] == peaks[1]
+    assert torch.equal(grads[1], grads[2])

@@ -94,3 +94,17 @@ def test_arrays_are_made_on_the_stream_of_the_call(device):
         back = [out[0], *out[1]] if name == "tsn_cg_unrolled" else out
         recorded = {e[1:] for e in device.log if e[0] == "record"}
         assert {(t.data_ptr(), "main") for t in back} | {(t.data_ptr(), "side") for t in ins} == recorded
+
+
+@pytest.mark.parametrize("checkpoint", [4, 50, 1 << 40])
+def test_interval_beyond_the_solve_costs_no_memory(device, checkpoint):
+    """A segment holds at most the solve's steps: an interval beyond them allocates what the solve's
+    own length does and reaches the library as that."""
+    plan, args = _plan(), _arguments(4, checkpoint)
+    _, saved = plan.cg_unrolled(*args)
+    plan.cg_unrolled_adjoint(saved, args[3], None, 1e-4, 4, checkpoint, _img(), _img(C))
+    work = [e[2].numel() for e in device.log if e[0] == "empty" and e[2].dtype == torch.uint8]
+    n = N * N
+    assert work == [8 * 7 * n + 8 * 296, 8 * n * (3 * 4 + 3 + (4 + 1) * C) + 8 * (2 * 296 + 2)]
+    for name in ("tsn_cg_unrolled", "tsn_cg_unrolled_adjoint"):
+        assert [e for e in device.log if e[0] == name][0][2][4:6] == (4, 4)

@@ -1471,7 +1471,8 @@ tsn_status tsn_cg_unrolled_adjoint(tsn_plan* plan, const void* smaps, const floa
     need_views(plan, true, true);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const bool pdl = direct_pdl(s);
-    const int64_t n = image_pixels(plan), cn = plan->C * n, cp = checkpoint;
+    const int64_t n = image_pixels(plan), cn = plan->C * n;
+    const int64_t cp = std::min(checkpoint, iters);  // a segment is at most the whole solve
     const float2 *st = static_cast<const float2*>(states), *qs = static_cast<const float2*>(q);
     const float2* ts = static_cast<const float2*>(coil_images);
     // work: p [cp + 1], r' [cp], q [cp], then q-bar, M q-bar, and with maps t [cp][C], t-bar [C]

@@ -316,6 +316,7 @@ class Plan:
                 x, saved = self.cg_unrolled(x0, r0, rho0, smaps, density, lam, iters, checkpoint, coils)
             _record(cur, x, *saved)
             return x, saved
+        checkpoint = min(checkpoint, iters)  # a segment is at most the whole solve
         cf, dev, shape = torch.complex64, r0.device, self.image_shape
         for t, name in ((x0, "x0"), (r0, "r0")):
             _dev_ptr(t, cf, shape, name)
@@ -346,6 +347,7 @@ class Plan:
                 out = self.cg_unrolled_adjoint(saved, smaps, density, lam, iters, checkpoint, xb, sb)
             _record(cur, *out)
             return out
+        checkpoint = min(checkpoint, iters)
         cf, dev, shape = torch.complex64, xb.device, self.image_shape
         states, rho, gamma, q = saved[:4]
         sp = _dev_ptr(smaps, cf, self.maps_shape, "smaps")
