@@ -108,3 +108,28 @@ def test_interval_beyond_the_solve_costs_no_memory(device, checkpoint):
     assert work == [8 * 7 * n + 8 * 296, 8 * n * (3 * 4 + 3 + (4 + 1) * C) + 8 * (2 * 296 + 2)]
     for name in ("tsn_cg_unrolled", "tsn_cg_unrolled_adjoint"):
         assert [e for e in device.log if e[0] == name][0][2][4:6] == (4, 4)
+
+
+@pytest.mark.parametrize("change", ["iters", "checkpoint", "shape", "dtype", "strides", "conj", "no coil images"])
+def test_reverse_pass_checks_what_was_saved(device, change):
+    """Arrays saved by another solve, or changed since, are refused before the library reads them."""
+    plan, args = _plan(), _arguments(4, 2)
+    saved = list(plan.cg_unrolled(*args)[1])
+    iters, checkpoint = 4, 2
+    if change == "iters":
+        iters = 5
+    elif change == "checkpoint":
+        checkpoint = 1
+    elif change == "shape":
+        saved[3] = saved[3][:, :2].contiguous()
+    elif change == "dtype":
+        saved[1] = saved[1].to(torch.float32)
+    elif change == "strides":
+        saved[4] = saved[4].transpose(-1, -2)
+    elif change == "conj":
+        saved[0] = saved[0].conj()
+    else:
+        saved = saved[:4]
+    with pytest.raises((TypeError, ValueError)):
+        plan.cg_unrolled_adjoint(saved, args[3], None, 1e-4, iters, checkpoint, _img(), _img(C))
+    assert not [e for e in device.log if e[0] == "tsn_cg_unrolled_adjoint"]

@@ -349,7 +349,12 @@ class Plan:
             return out
         checkpoint = min(checkpoint, iters)
         cf, dev, shape = torch.complex64, xb.device, self.image_shape
-        states, rho, gamma, q = saved[:4]
+        seg, f64 = -(-iters // checkpoint), torch.float64
+        shapes = [("states", cf, (seg, 3) + shape), ("rho", f64, (iters + 1,)), ("gamma", f64, (iters,)),
+                  ("q", cf, (seg,) + shape), ("coil images", cf, (seg,) + self.maps_shape)]
+        if sb is not None and len(saved) < 5:
+            raise ValueError("the map cotangent needs a solve that saved its coil images (coils=True)")
+        ptrs = [_dev_ptr(v, dt, sh, f"saved {name}") for v, (name, dt, sh) in zip(saved, shapes)]
         sp = _dev_ptr(smaps, cf, self.maps_shape, "smaps")
         dp = None if density is None else _dev_ptr(density, torch.float32, (self.samples,), "density")
         xp = _dev_ptr(xb, cf, shape, "xb")
@@ -360,9 +365,9 @@ class Plan:
         rb, pb = torch.zeros_like(xb), torch.zeros_like(xb)
         rhob = torch.zeros(2, dtype=torch.float64, device=dev)
         at = lambda v: C.c_void_p(v.data_ptr())
-        check(lib().tsn_cg_unrolled_adjoint(self._h, sp, dp, float(lam), int(iters), int(checkpoint), at(states), at(rho),
-                                            at(gamma), at(q), at(saved[4]) if sb is not None else None, xp, at(rb), at(pb),
-                                            bp, at(rhob), at(work), _stream_handle()))
+        check(lib().tsn_cg_unrolled_adjoint(self._h, sp, dp, float(lam), int(iters), int(checkpoint), *ptrs[:4],
+                                            ptrs[4] if sb is not None else None, xp, at(rb), at(pb), bp, at(rhob),
+                                            at(work), _stream_handle()))
         return rb, pb, rhob[iters & 1]
 
     def cg_sense(self, y, smaps, *, density=None, lam=1e-4, iters=10, operator_scale=1.0, out=None, stream=None,
