@@ -11,6 +11,7 @@ torch = pytest.importorskip("torch")
 
 from torch.overrides import TorchFunctionMode  # noqa: E402
 
+from trajsparsenufft_b200 import autograd as tad  # noqa: E402
 from trajsparsenufft_b200 import operator as op  # noqa: E402
 
 N, C, M = 4, 4, 10
@@ -133,3 +134,13 @@ def test_reverse_pass_checks_what_was_saved(device, change):
     with pytest.raises((TypeError, ValueError)):
         plan.cg_unrolled_adjoint(saved, args[3], None, 1e-4, iters, checkpoint, _img(), _img(C))
     assert not [e for e in device.log if e[0] == "tsn_cg_unrolled_adjoint"]
+
+
+def test_start_image_may_be_a_conjugated_view(device):
+    """The step-by-step solve starts from a copy of x0, which resolves a lazy conjugation; so does the
+    native one (tad.PlanOps)."""
+    args = _arguments(3, 2)
+    want = torch.complex(torch.rand(N, N), torch.rand(N, N))
+    for view in (want.conj().resolve_conj().conj(), want.T.contiguous().T):
+        states = tad.PlanOps(_plan()).unrolled(view, *args[1:])[1][0]
+        assert torch.equal(states[0, 0], want)

@@ -70,8 +70,8 @@ class PlanOps:
 
     def unrolled(self, x0, r0, rho0, smaps, density, lam, iters, checkpoint, coils):
         """All CG steps in one call: (x, tensors for unrolled_adjoint)."""
-        return self.plan.cg_unrolled(x0.contiguous(), r0.contiguous(), rho0, smaps.contiguous(), density, lam, iters,
-                                     checkpoint, coils)
+        return self.plan.cg_unrolled(x0.resolve_conj().contiguous(), r0.contiguous(), rho0, smaps.contiguous(), density,
+                                     lam, iters, checkpoint, coils)
 
     def unrolled_adjoint(self, saved, smaps, density, lam, iters, checkpoint, xb, sb):
         """All reverse steps in one call: (rb, pb, rhob) at the start, sb in place."""
