@@ -124,3 +124,88 @@ def test_forward_and_adjoint_vjps_match_autograd():
     got = torch.autograd.grad((tad.nufft_adjoint(ym, sm, ops) - xt).abs().pow(2).sum(), (ym, sm))
     for a, b in zip(got, ref):
         assert _rel(a, b) <= 1e-10
+
+
+class DensePlanOps(tad.PlanOps):
+    """PlanOps with every step-wise piece overridden (dense FP64) and the calls counted; the native
+    loops that it inherits would not run these pieces."""
+
+    def __init__(self, traj, n, plan=None):
+        super().__init__(plan)
+        self.dense, self.calls = DenseOps(traj, n), 0
+
+    def forward_coils(self, ci):
+        return self.dense.forward_coils(ci)
+
+    def adjoint_coils(self, y):
+        return self.dense.adjoint_coils(y)
+
+    def normal(self, p, smaps, density, lam, coils=False, pq=False, p_parts=None):
+        self.calls += 1
+        y = self.forward_coils(smaps * p)
+        t = self.adjoint_coils(y if density is None else y * density)
+        q = (smaps.conj() * t).sum(0) + lam * p
+        return q, t if coils else None, self.rdot(p, q) if pq else None
+
+    def rdot(self, a, b):
+        return (a.conj() * b).real.sum()
+
+    def forward_maps(self, x, smaps):
+        return self.forward_coils(smaps * x)
+
+    def step(self, rho, gamma, x, p, r, q):
+        r_n = r - (rho / gamma) * q
+        rho_n = self.rdot(r_n, r_n)
+        return None if x is None else x + (rho / gamma) * p, r_n, r_n + (rho_n / rho) * p, rho_n, None
+
+    def adjoint_step(self, rho, rho_n, gamma, rhob, rb, pb, p, q, r_n, xb):
+        alpha, betab = rho / gamma, self.rdot(pb, p)
+        rhob_n = rhob + betab / rho
+        rb += pb + 2.0 * rhob_n * r_n
+        alphab = self.rdot(xb, p) - self.rdot(rb, q)
+        gammab = -alphab * rho / gamma ** 2
+        pb *= rho_n / rho
+        pb += alpha * xb + gammab * q
+        return gammab * p - alpha * rb, -betab * rho_n / rho ** 2 + alphab / gamma, None
+
+    def adjoint_finish(self, pb, mqb, qb=None, t=None, tb=None, p=None, sb=None):
+        pb += mqb
+        if sb is not None:
+            sb += qb.conj() * t + tb * p.conj()
+
+
+def test_overridden_pieces_of_a_plans_ops_are_the_ones_that_run():
+    """A subclass of PlanOps that overrides a piece runs it in every step of the solve and of the
+    reverse pass: gradients against torch's own, 9 applications of M forward and back for 4 steps in
+    segments of 2 (the start, the steps, a recomputed one per segment, the reverse steps, x0)."""
+    _, y, smaps, x0, xt, w = _case(seed=11)
+    ops = DensePlanOps(synth.golden_radial(6, 2 * N), N)
+    leaves = [t.clone().requires_grad_(True) for t in (y, smaps, x0)]
+    ref = torch.autograd.grad((_plain_cg(*leaves, w, ops, 0.3, 4) - xt).abs().pow(2).sum(), leaves)
+    mine = [t.clone().requires_grad_(True) for t in (y, smaps, x0)]
+    x = tad.cg_sense(mine[0], mine[1], ops, x0=mine[2], density=w, lam=0.3, iters=4, checkpoint=2)
+    got = torch.autograd.grad((x - xt).abs().pow(2).sum(), mine)
+    assert ops.calls == 1 + 4 + 2 + 4 + 1
+    for name, a, b in zip(("y", "smaps", "x0"), got, ref):
+        assert _rel(a, b) <= 1e-9, name
+
+
+@pytest.mark.parametrize("where", ["ops class", "ops object", "plan class", "plan object", "nowhere"])
+def test_native_loops_stand_for_unchanged_pieces_only(where):
+    """The native loops replace PlanOps' own pieces over Plan's own methods, and no others."""
+    from trajsparsenufft_b200.operator import Plan
+
+    class OtherPlan(Plan):
+        def cg_step(self, *args, **kw):
+            return super().cg_step(*args, **kw)
+
+    class OtherOps(tad.PlanOps):
+        def normal(self, *args, **kw):
+            return super().normal(*args, **kw)
+
+    ops = (OtherOps if where == "ops class" else tad.PlanOps)(object.__new__(OtherPlan if where == "plan class" else Plan))
+    if where == "ops object":
+        ops.rdot = lambda a, b: None
+    if where == "plan object":
+        ops.plan.normal = lambda *args, **kw: None
+    assert tad._native(ops) == (where == "nowhere")

@@ -29,6 +29,8 @@ from __future__ import annotations
 
 import torch
 
+from .operator import Plan
+
 
 class PlanOps:
     """Coil-wise NUFFT pieces from a GPU plan (FP16x2 sparse interpolation, FP32 FFTs)."""
@@ -80,6 +82,23 @@ class PlanOps:
     def adjoint_finish(self, pb, mqb, qb=None, t=None, tb=None, p=None, sb=None):
         """pb += M qb and the coil-map cotangent update, in place."""
         self.plan.cg_adjoint_finish(pb, mqb, qb, t, tb, p, sb)
+
+
+def _is_own(obj, cls, names):
+    return all(getattr(getattr(obj, k, None), "__func__", None) is getattr(cls, k) for k in names)
+
+
+def _native(ops) -> bool:
+    """Whether the solve's steps may run in the native loops (`unrolled`, `unrolled_adjoint`).
+    PlanOps' loops stand for its own pieces over Plan's own methods: an ops object or a plan that
+    overrides one of these gets the step-by-step solve, which calls it."""
+    if not (hasattr(ops, "unrolled") and hasattr(ops, "unrolled_adjoint")):
+        return False
+    if getattr(ops.unrolled, "__func__", None) is not PlanOps.unrolled:
+        return True
+    return (_is_own(ops, PlanOps, ("normal", "rdot", "step", "adjoint_step", "adjoint_finish", "unrolled_adjoint")) and
+            _is_own(ops.plan, Plan, ("normal", "rdot", "cg_step", "cg_adjoint_step", "cg_adjoint_finish", "cg_unrolled",
+                                     "cg_unrolled_adjoint")))
 
 
 def _rdot(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
@@ -212,7 +231,7 @@ class UnrolledCgSense(torch.autograd.Function):
         b = S.combine(u)
         if x0_zero is None:                        # decided from the values (a host sync)
             x0_zero = not bool(x0.abs().amax() > 0)
-        if S.fused and iters > 0 and hasattr(ops, "unrolled"):  # every step in one native call
+        if S.fused and iters > 0 and _native(ops):  # every step in one native call
             r = b if x0_zero else b - S.M(x0)
             x, saved = ops.unrolled(x0, r, S.dot(r, r), smaps, density, lam, iters, checkpoint, ctx.needs_input_grad[1])
             ctx.ops, ctx.lam, ctx.iters, ctx.checkpoint, ctx.x0_zero = ops, lam, iters, checkpoint, x0_zero
