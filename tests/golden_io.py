@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import json
+import shutil
 from pathlib import Path
 
 import numpy as np
@@ -28,3 +29,13 @@ def read_dir(path: Path, names=PACK_FILES) -> dict[str, bytes]:
 
 def prod_input(name: str):
     return dict(np.load(GOLDEN / name / "input_csr.npz"))
+
+
+def shift_columns(src: Path, dst: Path, by: int) -> Path:
+    """A component directory whose columns all lie `by` further, behind as many unused ones."""
+    shutil.copytree(src, dst)
+    header = bytearray((dst / "header.bin").read_bytes())
+    header[20:24] = (int.from_bytes(header[20:24], "little") + by).to_bytes(4, "little")  # n_cols
+    (dst / "header.bin").write_bytes(bytes(header))
+    (np.fromfile(dst / "tile_col_ids.bin", dtype=np.int32) + np.int32(by)).tofile(dst / "tile_col_ids.bin")
+    return dst

@@ -382,3 +382,27 @@ def test_reference_steps_follow_the_reference_schedule():
     np.testing.assert_array_equal(x_plain.cpu().numpy(), x_again.cpu().numpy())
     with pytest.raises(TsnError, match="TSN_FLAG_REFERENCE_STEPS"):
         _plan("cfg0").cg_sense(yt, st, lam=1e-4, iters=10, scheduled_reference_period=2)
+
+
+def test_samples_beyond_32_bit_byte_offsets(tmp_path):
+    """An adjoint pack whose samples all lie behind 2^25 unused ones: at 16 coils their panel rows
+    start 4 GB in.  Component product and adjoint against the same pack without the unused samples:
+    the same coefficients and values, up to the power-of-two panel scale (FP16 high + residual keep
+    22 bits of it: 2^-21 between two scales, 1e-6 with room for the sums)."""
+    from golden_io import shift_columns
+    from trajsparsenufft_b200 import packing, synth
+    from trajsparsenufft_b200.operator import Plan
+    traj, n, g, c, ahead = synth.golden_radial(4, 32), 64, 128, 16, 1 << 25
+    dirs = packing.export_production(traj, tmp_path, im_size=n, grid_size=g, width=4)["G_T"]
+    far = [shift_columns(dirs / comp, tmp_path / f"far_{comp}", ahead) for comp in ("real", "imag")]
+    near = [dirs / "real", dirs / "imag"]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    y = torch.randn((c, ahead + len(traj)), dtype=torch.complex64, device="cuda", generator=gen)
+    dense = torch.randn((ahead + len(traj), 16), dtype=torch.float16, device="cuda", generator=gen)
+    got = []
+    for packs, first in ((near, ahead), (far, 0)):
+        plan = Plan.from_pack(None, None, *packs, im_size=n, grid_size=g, coils=c, width=4)
+        product = plan.interp_component("G_T", 1, dense[first:].contiguous())
+        got.append((plan.adjoint(y[:, first:].contiguous()), product))
+    assert rel_l2(got[1][0].cpu(), got[0][0].cpu()) <= 1e-6
+    assert torch.equal(got[1][1], got[0][1])

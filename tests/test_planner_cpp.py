@@ -11,7 +11,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
-from golden_io import GOLDEN, PACK_FILES, csr_view, layout_packs, prod_input, read_dir
+from golden_io import GOLDEN, PACK_FILES, csr_view, layout_packs, prod_input, read_dir, shift_columns
 from oracle import kb as okb
 from oracle import layout as olayout
 from oracle import planner as P
@@ -186,3 +186,23 @@ def test_plan_from_pack_rejects_bad_header(tmp_path):
     with pytest.raises(_lib.TsnError) as e:
         Plan.from_pack(str(src), str(other), None, None, im_size=16, grid_size=32, coils=4, width=6)
     assert e.value.kind == "FORMAT"
+
+
+@pytest.mark.parametrize("coils,columns,kind", [(16, (1 << 29) + 1, "UNSUPPORTED"), (12, 715827884, "UNSUPPORTED"),
+                                                (16, 1 << 29, "CUDA"), (12, 715827883, "CUDA"), (4, (1 << 31) - 1, "CUDA")])
+def test_columns_beyond_the_records_offsets_are_refused(tmp_path, coils, columns, kind):
+    """An adjoint pack alone may have any number of samples as columns; the records address 2^32
+    units of 16 bytes (2 coils' share of a panel row), and a pack beyond them is refused on the host.
+    The largest that fits passes that check and is stopped only by the missing GPU."""
+    import torch
+    from trajsparsenufft_b200.operator import Plan
+    if kind == "CUDA" and torch.cuda.is_available():
+        pytest.skip("a plan of this size would be made")
+    dirs = []
+    for comp in ("real", "imag"):
+        d = GOLDEN / "prod_radial16_fast" / "G_T" / comp
+        last = int(np.fromfile(d / "tile_col_ids.bin", dtype=np.int32).max())
+        dirs.append(shift_columns(d, tmp_path / comp, columns - 1 - last))
+    with pytest.raises(_lib.TsnError) as e:
+        Plan.from_pack(None, None, *dirs, im_size=16, grid_size=32, coils=coils, width=6)
+    assert e.value.kind == kind

@@ -28,11 +28,11 @@ struct CgState {
 
 // Interpolation view on the device: AoS tile records, in the order the persistent warps
 // stream them (warp w owns records [warp_ranges[w].x, warp_ranges[w].y))
-//   [0,128)                  u32 byte offset of each gathered panel row, in lane order: entry j
-//                            of lane group q (gather_lanes lanes) is at q * gather_lanes + j
-//                            and stands for tile column gather_column(rowh, q, j);
-//                            kGatherDead = dead column (all coefficients zero: zero-filled,
-//                            never read)
+//   [0,128)                  u32 offset of each gathered panel row in 16-byte units (even: rows
+//                            are multiples of 32 bytes), in lane order: entry j of lane group
+//                            q (gather_lanes lanes) is at q * gather_lanes + j and stands for
+//                            tile column gather_column(rowh, q, j); kGatherDead = dead column
+//                            (all coefficients zero: zero-filled, never read)
 //   [128+576c, +512)         f16 compressed A of component c as mma.sp fragments: lane l holds
 //                            A[l / 4 + 8 (i & 1)][8 (i >> 1) + 2 (l % 4) ..+1], i < 4, at 16 l
 //   [640+576c, +64)          u32 mma.sp pair metadata of component c, [16]
@@ -61,8 +61,10 @@ struct RecordInfo {
   int32_t chunk;       // chunk index | nchunks << 16
 };
 static_assert(sizeof(RecordInfo) == 16, "record info is 16 bytes");
-constexpr uint32_t kGatherDead = 16;  // offsets are multiples of 32: the bit is free, and the
-                                      // address it makes is inside the panel, though never read
+constexpr uint32_t kGatherDead = 1;  // offsets are even: the bit is free, and the address it makes
+                                     // is inside the panel, though never read
+// record offset of panel row `row` (of 2 rowh bytes)
+__host__ __device__ constexpr int64_t gather_offset(int rowh, int64_t row) { return row * (rowh / 8); }
 // Lanes that share a gathered row of 2 rowh bytes, and so the rows each lane gathers: a whole
 // row of 16-byte chunks when that is a power of two, else a 32-byte sector of it.
 __host__ __device__ constexpr int gather_lanes(int rowh) { return rowh == 48 ? 2 : rowh / 8; }

@@ -358,6 +358,16 @@ void build_tc_steps(tsn_plan* P, DevView& d, const HostView& h, bool rows_are_ce
   d.use_tc = true;
 }
 
+// Refuses a view whose gathered rows lie beyond the records' 32-bit offsets (a 64 GB panel: 2^29
+// rows of 16 coils). Only a pack of one view alone can have that many columns; the rows of the
+// other view are at most kMaxInterpRows.
+void check_gathers(const HostView& h, int coils, bool cols_are_cells) {
+  int64_t last = cols_are_cells ? h.n_cols - 1 : 0;
+  for (size_t i = 0; !cols_are_cells && i < h.tile_col_ids.size(); ++i) last = std::max<int64_t>(last, h.tile_col_ids[i]);
+  if (gather_offset(4 * coils, last) > static_cast<int64_t>(UINT32_MAX))
+    fail(TSN_ERR_UNSUPPORTED, "too many columns for 32-bit record offsets");
+}
+
 // Uploads one view into P->view[which], or into `target` (the reference-step views, which
 // leave the plan's info and the tensor-core stream alone).
 void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells, bool cols_are_cells,
@@ -439,7 +449,7 @@ void upload_view(tsn_plan* P, int which, const HostView& h, bool rows_are_cells,
           int64_t c = h.tile_col_ids[static_cast<size_t>(t) * kKTile + col];
           if (cols_are_cells) c = to_internal(P, c);
           if (cols_are_cells && ((live >> col) & 1u)) P->used[static_cast<size_t>(c)] = 1;
-          offsets[q * lanes + j] = ((live >> col) & 1u) ? static_cast<uint32_t>(c * rowh * 2) : kGatherDead;
+          offsets[q * lanes + j] = ((live >> col) & 1u) ? static_cast<uint32_t>(gather_offset(rowh, c)) : kGatherDead;
         }
       std::memcpy(r, offsets, sizeof offsets);
       for (int c = 0; c < ncomp; ++c) {
@@ -863,6 +873,8 @@ tsn_status tsn_plan_create_from_pack(const char* fwd_real, const char* fwd_imag,
     if (fwd_real && adj_real && hv[0].a.size() != hv[1].a.size())
       fail(TSN_ERR_FORMAT, "forward and adjoint packs have different component counts");
     P->ncomp = static_cast<int>((fwd_real ? hv[0] : hv[1]).a.size());
+    if (fwd_real) check_gathers(hv[0], P->C, true);
+    if (adj_real) check_gathers(hv[1], P->C, false);
     CUDA_OK(cudaSetDevice(desc->device));  // all host-side checks are done: touch the device now
     std::vector<float> sc(static_cast<size_t>(P->N) * P->N);
     if (scaling) {
@@ -1904,7 +1916,8 @@ tsn_status tsn_interp_component(tsn_plan* plan, int32_t view, int32_t component,
         for (int q = 0; q < kKTile / lanes; ++q)
           for (int j = 0; j < lanes; ++j) {
             const uint32_t o = in[q * lanes + j];
-            cols[gather_column(rowh, q, j)] = o == kGatherDead ? o : o / static_cast<uint32_t>(rowh * 2) * 32;
+            cols[gather_column(rowh, q, j)] =
+                o == kGatherDead ? o : static_cast<uint32_t>(gather_offset(16, o / gather_offset(rowh, 1)));
           }
         for (int q = 0; q < kKTile / lanes16; ++q)
           for (int j = 0; j < lanes16; ++j) out16[q * lanes16 + j] = cols[gather_column(16, q, j)];
