@@ -406,3 +406,24 @@ def test_samples_beyond_32_bit_byte_offsets(tmp_path):
         got.append((plan.adjoint(y[:, first:].contiguous()), product))
     assert rel_l2(got[1][0].cpu(), got[0][0].cpu()) <= 1e-6
     assert torch.equal(got[1][1], got[0][1])
+
+
+# The row stages' forms in a solve: forward rows with the fused update and inverse rows with four
+# partial sums whose map rows are staged in shared memory (8 coils on 1024 points: an image row of
+# 476 is the last that is, with 480 two CTAs no longer fit on an SM) and lines that read them from
+# global memory (16 coils on 640 points, 12 on 1024).
+@pytest.mark.parametrize("n,g,c", [(256, 640, 16), (320, 640, 16), (476, 1024, 8), (480, 1024, 8), (412, 1024, 12)])
+def test_solve_on_long_lines(n, g, c):
+    """Three iterations (a plain first step, two fused updates, the last update) against the FP16
+    coefficients' CG in FP64: seven operator applications, each within the operator's 2e-5."""
+    from trajsparsenufft_b200 import synth
+    from trajsparsenufft_b200.operator import Plan
+    traj = synth.golden_radial(24, 512)
+    x, s = synth.ellipse_phantom(n, 5), synth.coil_maps(n, c, 5)
+    emu = oop.KbSenseOperator(traj, n, g, 4, matrix_mode="fp16", workers=8)
+    y = np.ascontiguousarray(emu.forward(x, s), dtype=np.complex64)
+    want, _, _ = oop.cg_sense(lambda v: emu.forward(v, s), lambda v: emu.adjoint(v, s), y, 3, 1e-4)
+    plan = Plan.from_trajectory(traj, im_size=n, grid_size=g, coils=c, width=4)
+    got, _, _ = plan.cg_sense(torch.from_numpy(y).cuda(), torch.from_numpy(s).cuda(), lam=1e-4, iters=3)
+    err = rel_l2(got.cpu().numpy(), want)
+    assert err <= 7 * 2e-5, err

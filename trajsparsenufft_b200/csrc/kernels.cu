@@ -557,6 +557,8 @@ __device__ __forceinline__ void cp_async_bytes(void* dst, const void* src, int b
 #define TSN_FFT_BOUNDS(T) __launch_bounds__((T), (1024 / (T)) > 0 ? 1024 / (T) : 1)
 #define TSN_ROW_BOUNDS(T) __launch_bounds__((T), (T) <= 256 ? 768 / (T) : (T) <= 640 ? 2 : 1)
 
+constexpr int kRowRed = 132;  // doubles of the row stages' static array (sums of partials)
+
 // Lines of more than 256 threads (12 and 16 coils, large grids) leave the last inverse
 // butterflies in shared memory instead of holding them in registers while the region changes
 // hands: two CTAs of 480-640 threads then stay resident per SM, where one CTA per SM took three
@@ -617,7 +619,7 @@ fwd_rows_kernel(FftArgs f, const float2* __restrict__ x, float2* __restrict__ z1
   float* srow = reinterpret_cast<float*>(row3 + (mode == 4 ? N : 0));
   float2* maps_s = reinterpret_cast<float2*>(srow + N);
   const int pitch = map_pitch(N);
-  __shared__ double red[132];
+  __shared__ double red[kRowRed];
   const int tid = threadIdx.x, c = tid % C;
   // part 1: rows no kernel of a solve writes (coil maps, deapodization); part 2: the rest
   const int i0 = blockIdx.x;
@@ -939,7 +941,7 @@ inv_rows_kernel(FftArgs f, const float2* __restrict__ w1, float2* __restrict__ o
   float2* errow = eprow + (mode >= 2 ? N : 0);
   const float2* rsrc = mode == 2 ? r : mode == 3 ? x : nullptr;  // r, or the right-hand side b
   float* escale = reinterpret_cast<float*>(errow + (rsrc ? N : 0));
-  __shared__ double red[132];
+  __shared__ double red[kRowRed];
   const int tid = threadIdx.x, c = tid % C;
   // part 1: rows no kernel of a solve writes (coil maps, deapodization); part 2: the rest
   const int i0 = blockIdx.x;
@@ -1135,8 +1137,11 @@ static size_t fft_rows_bytes() {
   return sizeof(float2) * static_cast<size_t>(LineFft<G, C, false>::ROWS) * C;
 }
 // The row stages stage their coil-map rows (and other epilogue rows) in shared memory while
-// two CTAs still fit on an SM with them; larger lines read them from global memory.
-constexpr size_t kFftStageSmem = 114 * 1024;
+// two CTAs still fit on an SM with them (half of its 228 KB, less the 1 KB that each CTA reserves
+// and the kernel's static array); larger lines read them from global memory. Lines of 112-114 KB
+// staged, one CTA per SM, and not, two of them: adjoint of 256^2 x 16 coils on 640 points 66.9 and
+// 65.0 us, 6-iteration solve of 488^2 x 8 coils on 1024 points 945 and 919 us.
+constexpr size_t kFftStageSmem = 228 * 1024 / 2 - 1024 - kRowRed * sizeof(double);
 
 // Dynamic shared memory beyond the default 48 KB, of which the kernels' static arrays take up
 // to 2 KB, has to be asked for.
