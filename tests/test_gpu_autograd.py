@@ -340,3 +340,24 @@ def test_interval_beyond_the_solve_costs_no_memory():
         grads.append(sm.grad)
     assert peaks[2] == peaks[1]
     assert torch.equal(grads[1], grads[2])
+
+
+@pytest.mark.parametrize("iters,checkpoint,need_s,start", [(3, 2, True, False), (4, 3, False, True)])
+def test_native_unrolled_solve_of_a_volume(iters, checkpoint, need_s, start):
+    """The native loops of a volume, whose partial sums are settled in kernels of their own, against
+    the step-wise path: FP32 rounding grown by the solve, as for images."""
+    from gpu_cases import volume_case, volume_measurement
+    from trajsparsenufft_b200 import autograd as tad
+    from trajsparsenufft_b200.operator import Plan
+    traj, x, s, n, g, c, j = volume_case("vol64")
+    plan = Plan.from_trajectory(traj, im_size=n, grid_size=g, coils=c, width=j)
+    xt, st, yt = (torch.from_numpy(v).cuda() for v in (x, s, volume_measurement("vol64")))
+    got = []
+    for ops in (tad.PlanOps(plan), _StepOps(plan)):
+        y, sm = yt.clone().requires_grad_(True), st.clone().requires_grad_(need_s)
+        x0 = (0.3 * xt if start else torch.zeros_like(xt)).requires_grad_(True)
+        xk = tad.cg_sense(y, sm, ops, x0=x0, lam=1e-4, iters=iters, checkpoint=checkpoint)
+        (xk - xt).abs().pow(2).sum().backward()
+        got.append([v.detach() for v in (xk, y.grad, x0.grad) + ((sm.grad,) if need_s else ())])
+    for a, b in zip(*got):
+        assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b)) <= 1e-4
