@@ -427,3 +427,21 @@ def test_solve_on_long_lines(n, g, c):
     got, _, _ = plan.cg_sense(torch.from_numpy(y).cuda(), torch.from_numpy(s).cuda(), lam=1e-4, iters=3)
     err = rel_l2(got.cpu().numpy(), want)
     assert err <= 7 * 2e-5, err
+
+
+@pytest.mark.parametrize("coils", [8, 12, 16])
+def test_component_product_does_not_depend_on_the_coils(coils):
+    """The records' offsets are those of the plan's panel rows; the product takes 16-channel rows at
+    every coil count.  The same tiles in the same chunks: equal bits."""
+    from trajsparsenufft_b200.operator import Plan
+    root, out = GOLDEN / "prod_spiral32_opt", []
+    for c in (4, coils):
+        plan = Plan.from_pack(root / "G" / "real", root / "G" / "imag", root / "G_T" / "real", root / "G_T" / "imag",
+                              im_size=32, grid_size=64, coils=c, width=6)
+        out.append([])
+        for view in ("G", "G_T"):
+            for ci, comp in enumerate(("real", "imag")):
+                dense = np.fromfile(root / view / comp / "dense_input.bin", dtype=np.float16).reshape(-1, 16)
+                out[-1].append(plan.interp_component(view, ci, torch.from_numpy(dense).cuda()))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)

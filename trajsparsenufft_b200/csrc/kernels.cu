@@ -485,6 +485,36 @@ void launch_interp(const InterpView& v, const __half* panel, int rowh, bool spli
   }
 }
 
+// One warp per record, each lane an offset and 16-byte pieces of the rest. Bound by reading and
+// writing the records once; a rebuild on the host cost the 256^2 x 8-coil view 11 ms a call.
+__global__ void narrow_records_kernel(const uint8_t* __restrict__ records, int64_t tiles, int rowh, int ncomp,
+                                      int component, uint8_t* __restrict__ out) {
+  const int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t >= tiles) return;
+  const uint8_t* src = records + t * record_bytes(ncomp);
+  uint8_t* dst = out + t * record_bytes(1);
+  // entry `lane` of 16-channel rows stands for tile column col, which lane group q of the view's
+  // own rows holds as its entry j: col = q + j * (lane groups)
+  const int col = gather_column(16, lane / gather_lanes(16), lane % gather_lanes(16));
+  const int lanes = gather_lanes(rowh), groups = 32 / lanes;
+  const uint32_t f = reinterpret_cast<const uint32_t*>(src)[col % groups * lanes + col / groups];
+  reinterpret_cast<uint32_t*>(dst)[lane] =
+      f == kGatherDead ? f : static_cast<uint32_t>(gather_offset(16, f / static_cast<uint32_t>(gather_offset(rowh, 1))));
+  const uint4* comp = reinterpret_cast<const uint4*>(src + 128 + 576 * component);
+  uint4* to = reinterpret_cast<uint4*>(dst + 128);
+  to[lane] = comp[lane];                               // A
+  if (lane < 4) to[32 + lane] = comp[32 + lane];       // metadata
+  const uint4* info = reinterpret_cast<const uint4*>(src + 128 + 576 * ncomp);
+  if (lane < kRecInfoBytes / 16) to[36 + lane] = info[lane];
+}
+
+void launch_narrow_records(const uint8_t* records, int64_t tiles, int rowh, int ncomp, int component, uint8_t* out,
+                           cudaStream_t s) {
+  if (tiles <= 0) return;
+  narrow_records_kernel<<<static_cast<unsigned>((tiles + 7) / 8), 256, 0, s>>>(records, tiles, rowh, ncomp, component, out);
+}
+
 // ------------------------------------------------------------------------------------------
 // Reductions
 // ------------------------------------------------------------------------------------------

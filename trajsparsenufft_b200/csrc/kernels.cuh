@@ -143,6 +143,11 @@ inline bool fft_grid_supported(int g) {
 void launch_interp(const InterpView& v, const __half* panel, int rowh, bool split, int epi, bool conj,
                    const InterpOut& o, cudaStream_t s);
 
+// One component's records for 16-channel rows: `tiles` records of `ncomp` components whose offsets
+// are those of panel rows of 2 rowh bytes -> record_bytes(1) each, offsets of 32-byte rows.
+void launch_narrow_records(const uint8_t* records, int64_t tiles, int rowh, int ncomp, int component, uint8_t* out,
+                           cudaStream_t s);
+
 // ---- interpolation on tcgen05.mma.sp (real pack, 8 coils) ------------------------------------
 // Seven 16-row tiles are stacked into one M = 128 sparse A operand (rows 112..127 zero) and
 // their 32 gathered panel rows side by side into one N = 7 x 32 = 224 B operand; one

@@ -1900,35 +1900,11 @@ tsn_status tsn_interp_component(tsn_plan* plan, int32_t view, int32_t component,
     InterpOut o;
     o.raw = dout.as<float>();
     o.rows = d.output_size;
-    // single-component records (columns | A and metadata of the component | record info and
-    // rows) whose offsets are those of 16-channel rows
     DeviceBuffer narrow;
-    {
-      const int one_rec = record_bytes(1), rowh = 4 * plan->C, lanes = gather_lanes(rowh), lanes16 = gather_lanes(16);
-      std::vector<uint8_t> host(static_cast<size_t>(d.tiles) * d.v.rec_bytes);
-      CUDA_OK(cudaMemcpy(host.data(), d.v.records, host.size(), cudaMemcpyDeviceToHost));
-      std::vector<uint8_t> one(static_cast<size_t>(d.tiles) * one_rec);
-      for (int64_t t = 0; t < d.tiles; ++t) {
-        const uint8_t* src = &host[t * d.v.rec_bytes];
-        uint8_t* dst = &one[t * one_rec];
-        uint32_t in[kKTile], cols[kKTile], out16[kKTile];
-        std::memcpy(in, src, sizeof in);
-        for (int q = 0; q < kKTile / lanes; ++q)
-          for (int j = 0; j < lanes; ++j) {
-            const uint32_t o = in[q * lanes + j];
-            cols[gather_column(rowh, q, j)] =
-                o == kGatherDead ? o : static_cast<uint32_t>(gather_offset(16, o / gather_offset(rowh, 1)));
-          }
-        for (int q = 0; q < kKTile / lanes16; ++q)
-          for (int j = 0; j < lanes16; ++j) out16[q * lanes16 + j] = cols[gather_column(16, q, j)];
-        std::memcpy(dst, out16, sizeof out16);
-        std::memcpy(dst + 128, src + 128 + 576 * component, 576);
-        std::memcpy(dst + 128 + 576, src + 128 + 576 * d.v.ncomp, kRecInfoBytes);
-      }
-      narrow.upload(one);
-      v.records = narrow.as<uint8_t>();
-      v.rec_bytes = one_rec;
-    }
+    narrow.alloc(static_cast<size_t>(d.tiles) * record_bytes(1));
+    launch_narrow_records(d.v.records, d.tiles, plan->rowh, d.v.ncomp, component, narrow.as<uint8_t>(), s);
+    v.records = narrow.as<uint8_t>();
+    v.rec_bytes = record_bytes(1);
     v.ncomp = 1;
     launch_interp(v, din.as<__half>(), 16, false, EPI_RAW, false, o, s);
     launch_gather_rows_f32(dout.as<float>(), rm.as<int32_t>(), d.output_size, 16, out, s);
