@@ -110,7 +110,8 @@ def _rdot(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 
 
 class _Sense:
-    """SENSE algebra over a CoilOps object (no autograd inside).  When the ops object has
+    """SENSE algebra over a CoilOps object (no autograd inside), for the step-by-step solve and the
+    operators around a native one (_native).  When the ops object has
     `normal` and `rdot` (PlanOps), M p, its coil images and the FP64 inner products run in the
     plan's CUDA kernels; otherwise they are composed here from forward_coils / adjoint_coils."""
 

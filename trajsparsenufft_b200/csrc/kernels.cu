@@ -30,8 +30,9 @@ using namespace dev;
 // Inside the solver's graph only the interpolation is launched so: a plain graph edge costs
 // 0.65 us, and FFT stages that start early wait beside a kernel that leaves room on the SMs
 // (10-iteration solves, plain / programmatic FFT stages: 256^2 x 8 coils 616 / 636 us, 128^2 x
-// 4 coils 302 / 309 us). The kernel ahead of an interpolation calls pdl_trigger after its own
-// wait; the others leave it to their end. Batched cases, whose kernels run side by side on
+// 4 coils 302 / 309 us). The column stage ahead of a forward interpolation and the interpolation
+// ahead of an adjoint one call pdl_trigger after their own wait; the others (split_samples among
+// them, ahead of a plain adjoint's interpolation) leave it to their end. Batched cases, whose kernels run side by side on
 // slices of the GPU, launch everything plainly: early CTAs would wait beside the other cases'
 // kernels (the 48-case batch measured 1191 recons/s with it, 1325-1390 without it).
 //
@@ -217,10 +218,9 @@ __device__ __forceinline__ void interp_finish_item(float (&acc)[NCOMP][NA][4], c
   }
 }
 
-//
 // What bounds it: instruction issue and the latency of the chain record -> gather -> MMA; with
 // both data streams left out a launch still takes three quarters of its time. So the record
-// holds what a lane needs as the lane needs it (the byte offsets of its gathers in one shared
+// holds what a lane needs as the lane needs it (the offsets of its gathers in one shared
 // load, A as MMA fragments) instead of column ids that were passed around by shuffles and
 // tested for every 16-byte copy (209 warp instructions per tile). 10-iteration solves: 256^2
 // with 8 coils 615 -> 594 us, with 16 coils 1210 -> 1009 us, 128^2 with 4 coils 343 -> 322 us.

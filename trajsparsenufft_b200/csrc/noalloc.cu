@@ -67,7 +67,7 @@ std::mutex g_setup_mutex;
   tsn::fail(TSN_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-DeviceSetup& setup_device(int device, cudaStream_t s) {
+DeviceSetup& setup_device(int device) {
   if (device < 0 || device >= kMaxDevices) tsn::fail(TSN_ERR_UNSUPPORTED, "device ordinal out of range");
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   DeviceSetup& d = g_setup[device];
@@ -129,7 +129,7 @@ extern "C" tsn_status tsn_fft_adjoint_image_static(int32_t im_size, int32_t grid
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) cuda_fail(e, "cudaGetDevice");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    DeviceSetup& d = setup_device(device, s);
+    DeviceSetup& d = setup_device(device);
     tsn::FftArgs f;
     f.N = im_size;
     f.G = grid_size;

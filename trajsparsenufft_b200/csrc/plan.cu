@@ -12,7 +12,6 @@
 #include <iterator>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -576,7 +575,7 @@ void setup_tc(tsn_plan* P) {
     if (d.present && d.use_tc) d.tc.error = P->tc_error.as<int32_t>();
 }
 
-// FFT endpoints are built for power-of-two grids of 128..1024 points.
+// FFT endpoints are built for the grid sizes of fft_grid_supported.
 void need_fft(const tsn_plan* P) {
   const int G = P->G;
   if (!fft_grid_supported(G))
@@ -967,7 +966,7 @@ tsn_status tsn_plan_create_from_trajectory(const float* traj, int64_t m, const t
       upload_view(P.get(), TSN_VIEW_GT, hv[1], true, false);
       hv[1] = HostView();
       upload_gaps(P.get());
-    allocate_workspaces(P.get());
+      allocate_workspaces(P.get());
       setup_tc(P.get());
       P->info.samples = P->M;
       P->info.im_size = P->N;
