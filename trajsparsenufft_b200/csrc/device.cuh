@@ -62,10 +62,17 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 __device__ __forceinline__ void cp_async16_u32(uint32_t smem_dst, const void* gmem_src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_dst), "l"(gmem_src) : "memory");
 }
-// 16-byte copy to a shared address (bytes = 16), or a 16-byte zero fill without a global read
-// (bytes = 0).
-__device__ __forceinline__ void cp_async16_zfill(uint32_t smem_dst, const void* gmem_src, uint32_t bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_dst), "l"(gmem_src), "r"(bytes) : "memory");
+// 16-byte copy to a shared address, or (skip != 0) a 16-byte zero fill without a global read.
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t smem_dst, const void* gmem_src, uint32_t skip) {
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; cp.async.cg.shared.global [%0], [%1], 16, p; }\n" ::"r"(smem_dst),
+               "l"(gmem_src), "r"(skip)
+               : "memory");
+}
+// base + 16 units, in one instruction
+__device__ __forceinline__ const uint8_t* offset16(const uint8_t* base, uint32_t units) {
+  uint64_t a;
+  asm("mad.wide.u32 %0, %1, 16, %2;" : "=l"(a) : "r"(units), "l"(base));
+  return reinterpret_cast<const uint8_t*>(a);
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>

@@ -321,12 +321,11 @@ __global__ void __launch_bounds__(kInterpWarps * 32, interp_ctas(ROWH, NCOMP)) i
       }
 #pragma unroll
       for (int i = 0; i < NOFF; ++i) {
-        const uint32_t bytes = (~f[i] & kGatherDead) << 4;  // 16, or 0 (zero fill, no read) for a dead column
-        const uint8_t* src = pb + static_cast<size_t>(f[i]) * 16;
+        const uint8_t* src = offset16(pb, f[i]);
 #pragma unroll
         for (int u = 0; u < NSUB; ++u)
-          cp_async16_zfill((CH == 8 && (i & 1) ? dst0 ^ 64u : dst0) + stage * STAGE + i * (32 / LPR) * BYTES + u * LPR * 16,
-                           src + u * LPR * 16, bytes);
+          cp_async16_or_zero((CH == 8 && (i & 1) ? dst0 ^ 64u : dst0) + stage * STAGE + i * (32 / LPR) * BYTES + u * LPR * 16,
+                             src + u * LPR * 16, f[i] & kGatherDead);
       }
     }
     cp_async_commit();
