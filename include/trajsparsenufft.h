@@ -264,7 +264,8 @@ tsn_status tsn_cg_adjoint_finish(tsn_plan* plan, int64_t n, int32_t coils, void*
 /* The steps of a differentiable unrolled solve, enqueued by one call each (the loops of
  * tsn_normal with tsn_cg_step, and of tsn_normal with tsn_cg_adjoint_step and _finish, without a
  * host call per step).  iters >= 1, checkpoint >= 1, segments = ceil(iters / checkpoint).
- * Images hold n complex64 (one plan image), device pointers 16-byte aligned.
+ * Images hold n complex64 (one plan image), device pointers 16-byte aligned (the cotangents xb,
+ * rb, pb and sb: 8).
  *
  * tsn_cg_unrolled runs `iters` iterations of M = A^H W A + lambda from x, r, p in states[0]:
  *   states       [segments][3][n]  x, r, p before iterations 0, checkpoint, 2 checkpoint, ...

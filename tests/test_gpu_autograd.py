@@ -361,3 +361,27 @@ def test_native_unrolled_solve_of_a_volume(iters, checkpoint, need_s, start):
         got.append([v.detach() for v in (xk, y.grad, x0.grad) + ((sm.grad,) if need_s else ())])
     for a, b in zip(*got):
         assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b)) <= 1e-4
+
+
+def test_gradient_at_an_8_byte_address():
+    """A loss that packs the image behind one more value hands the solve a gradient that is a contiguous
+    view 8 bytes off a 16-byte boundary: the same gradient as from a copy, bit for bit."""
+    from gpu_cases import torch_inputs
+    from trajsparsenufft_b200 import autograd as tad
+    from trajsparsenufft_b200.operator import Plan
+    traj, x, s, n, g, c, j, _ = case("small")
+    plan = Plan.from_trajectory(traj, im_size=n, grid_size=g, coils=c, width=j)
+    xt, st, yt = torch_inputs("small")
+    grads, seen = [], []
+    for packed in (False, True):
+        y, sm = yt.clone().requires_grad_(True), st.clone().requires_grad_(True)
+        xk = tad.cg_sense(y, sm, tad.PlanOps(plan), lam=LAM, iters=3, checkpoint=2)
+        flat = torch.empty(n * n + 1, dtype=torch.complex64, device="cuda")
+        flat[1:] = (xk.detach() - xt).reshape(-1)
+        gx = flat[1:].view(n, n)
+        seen.append(gx.data_ptr() % 16)
+        torch.autograd.backward(xk, gx if packed else gx.clone())
+        grads.append((y.grad, sm.grad))
+    assert seen == [8, 8]
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)

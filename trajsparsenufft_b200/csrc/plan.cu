@@ -1478,7 +1478,7 @@ tsn_status tsn_cg_unrolled_adjoint(tsn_plan* plan, const void* smaps, const floa
     if (sb && !coil_images) fail(TSN_ERR_ARG, "the map cotangent needs the coil images");
     if (iters < 1 || checkpoint < 1) fail(TSN_ERR_ARG, "iters and checkpoint must be >= 1");
     if (!std::isfinite(lambda)) fail(TSN_ERR_ARG, "lambda must be finite");
-    need_aligned({smaps, density, states, q, coil_images, xb, rb, pb, sb, work});
+    need_aligned({smaps, density, states, q, coil_images, work});  // the cotangents are read 8 bytes at a time
     need_views(plan, true, true);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const bool pdl = direct_pdl(s);
