@@ -212,7 +212,10 @@ def measured_peaks() -> tuple[float, str]:
     return 6650.0, "fallback"
 
 
-def committed_traffic(kernel: str):
+def committed_traffic(kernel: str, cfg: dict):
+    """Measured DRAM bytes of a launch of the headline configuration (None for the others)."""
+    if any(cfg[k] != v for k, v in CONFIGS["headline"].items()):
+        return None
     p = ROOT / "profiles" / "traffic.json"
     if p.exists():
         try:
@@ -413,7 +416,7 @@ def run_ours(args, cfg) -> dict:
         "gpu_launches": args.steps * (5 + 6 * iters + 2),
         "roofline": {"bound": "hbm", "kernel": dominant, "achieved": round(achieved, 1), "peak": peak,
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                     "traffic": committed_traffic(dominant),
+                     "traffic": committed_traffic(dominant, cfg),
                      "algorithmic_bytes_per_launch": alg[dominant], "launch_ms": round(stages[dominant], 5)},
         "step_roofline": {"algorithmic_bytes_per_recon": int(recon_bytes),
                           "achieved_GBs": round(recon_bytes * value / world / 1e9, 1),

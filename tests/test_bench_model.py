@@ -52,3 +52,9 @@ def test_numa_local_is_a_no_op_without_nvml_answer():
     info = numa.summary()
     assert info["allowed_cpus"] == len(before)
     assert info["pinned_on_gpu_node"] == bool(numa.cpus)
+
+
+def test_traffic_belongs_to_the_headline_configuration():
+    """The committed DRAM bytes are those of the headline's launches; other configurations have none."""
+    assert bench.committed_traffic("interp_fwd", dict(bench.CONFIGS["headline"])) > 0
+    assert bench.committed_traffic("interp_fwd", dict(bench.CONFIGS["cfg0"])) is None
