@@ -95,7 +95,7 @@ def test_inputs_rewritten_between_calls(volume):
             maps.neg_()
             put(1)
             out.append(plan.normal(img, maps, density=w, lam=1e-4, p_norm_parts=parts)[0])
-            for b in bufs:  # a late read of this round's inputs would see zeros
+            for b in bufs:  # a read that comes late would see zeros
                 b.zero_()
         torch.cuda.synchronize()
         runs.append(out)
